@@ -165,7 +165,14 @@ typedef struct wk_fit_desc {
    * cells near the relaxation limit) follow the FP64 trajectory closely;
    * runs the two-pass kernels (WK_KERNEL_TMA is refused).                  */
   int comp_stencil;
+  /* WK_SYNC_WORDS device words, zeroed once by the caller and used by one
+   * call at a time, for the grid barrier of the launch that runs all steps
+   * of a call on a small grid (WK_KERNEL_AUTO, steps_per_launch 0).  NULL:
+   * every step is launched by itself.  The results do not depend on it.    */
+  unsigned* sync;
 } wk_fit_desc;
+
+#define WK_SYNC_WORDS 96
 
 #define WK_KERNEL_AUTO 0   /* WK_KERNEL_TMA when its conditions hold, else
                               WK_KERNEL_TWOPASS when Nx, Ny, Nz >= 5, else

@@ -218,6 +218,47 @@ def test_schedules_equal_cell_kernel_with_beam_and_capture(kernel, tile):
     assert torch.equal(ha, hb)
 
 
+@pytest.mark.parametrize("shape", [(7, 5, 9), (16, 13, 40), (67, 9, 23), (33, 41, 57)])
+@pytest.mark.parametrize("idx", VALID)
+def test_many_steps_per_launch_equal_cell_kernel(idx, shape):
+    """One launch for all steps of a call (small grids) gives the fields and
+    the Ez history of the per-cell kernel value for value, on every face and
+    material mix, from random fields (wrapped neighbours and masks matter),
+    with the beam and the capture, an odd and an even number of steps, and
+    with the step index read from a device counter."""
+    from wakis_b200 import _native
+    from wakis_b200.sources import Beam
+    c = dict(cases.STEP_CASES[idx], shape=shape)
+    try:
+        a, b = b200_step_case(c), b200_step_case(c)
+    except ValueError:
+        pytest.skip("no cell with a finite relaxation time, as upstream")
+    b.kernel = "cell"
+    E0, H0 = cases.initial_fields(c, a.N)
+    bp = Beam(**c["beam"]).params(a)
+    hist = [torch.zeros((9, a.Nz, 16), dtype=a._cap_dtype, device="cuda") for _ in range(2)]
+    ctr = torch.full((1,), 9, dtype=torch.int64, device="cuda")
+    for s, h in zip((a, b), hist):
+        s._first_step()
+        s.E.fromarray(E0)
+        s.H.fromarray(H0)
+        cap = (h, 1, 1, 3, 3)
+        s._advance(9, 0, beam=bp, capture=cap)
+        if s is a and s._j_state != 2:
+            d = s._step_desc(beam=bp, capture=cap)
+            d.step_dev = ctr.data_ptr()
+            _native.check(s._lib.wk_fit_step(d, 6, 0, s._stream()), "wk_fit_step")
+            d.step_dev = None
+        else:
+            s._advance(6, 9, beam=bp, capture=cap)
+        s.check_status()
+    assert int(a._sync.abs().sum().item()) == 0
+    assert np.array_equal(a.E.numpy(), b.E.numpy())
+    assert np.array_equal(a.H.numpy(), b.H.numpy())
+    assert torch.equal(hist[0], hist[1])
+    assert np.abs(a.E.numpy()).max() > 0
+
+
 def _wake_errors(a, b):
     return {n: rel_err(getattr(a, n), getattr(b, n)) for n in ("WP", "WPx", "WPy", "Z", "Zx")}
 

@@ -15,6 +15,7 @@ WK_F64, WK_F32, WK_F32C = 0, 1, 2
 WK_J_ZERO, WK_J_SIGMA_E, WK_J_ARRAY = 0, 1, 2
 WK_KERNEL_AUTO, WK_KERNEL_CELL, WK_KERNEL_TWOPASS, WK_KERNEL_TMA = 0, 1, 4, 6
 WK_BATCH_PERSISTENT, WK_BATCH_PHASES = 0, 1
+WK_SYNC_WORDS = 96
 
 _vp = ctypes.c_void_p
 _i = ctypes.c_int
@@ -47,6 +48,7 @@ class FitDesc(ctypes.Structure):
         ("wait_ns", _ll),
         ("steps_per_launch", _i),
         ("comp_stencil", _i),
+        ("sync", _vp),
     ]
 
 

@@ -236,6 +236,14 @@ template <typename T>
 cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
                        int rows);
 
+// All steps of a call in one launch, for small grids (fit_loop.cu): the grid
+// fits the row factors kept in shared memory; every dimension >= 2.
+template <typename T>
+bool loop_supported(const FitParams<T>& p);
+template <typename T>
+cudaError_t launch_loop(const FitParams<T>& p, int n_steps, long long step0, unsigned* sync,
+                        cudaStream_t st);
+
 // Two steps per launch (fit_tma2.cu): k_tma2 covers grids whose faces are
 // all PEC-masked and clean, with J = 0 or sigma*E.
 template <typename T>

@@ -95,6 +95,21 @@ int run_fused(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_t s
   int par = d->par;
   const bool big = d->Nx >= 5 && d->Ny >= 5 && d->Nz >= 5 && d->Nz - 4 <= 65535 &&
                    (d->Ny - 4 + 1) / 2 <= 65535;
+  // small grids: all steps in one launch where the tiles fit the shared
+  // memory of the SMs (about 430k FP64 or 860k FP32 cells).  From 4 steps on
+  // it is the faster one over the whole range, set-up included: 4 steps of
+  // 16x16x24 FP64 25 against 42 us, 40x40x80 FP64 51 / 100, 55x61x110 FP64
+  // 102 / 189, 64x64x160 FP32 132 / 126; 8 steps 37 / 83, 79 / 199, 158 / 377,
+  // 192 / 251; 2 steps of 64x64x160 100 / 67.
+  if (d->kernel == WK_KERNEL_AUTO && big && d->sync && n_steps >= 4 && d->steps_per_launch == 0 &&
+      !g_kernel_timer) {
+    const FitParams<T> p = make_params<T>(d, par);
+    if (loop_supported<T>(p)) {
+      cudaError_t e = launch_loop<T>(p, n_steps, step0, d->sync, st);
+      if (e != cudaSuccess) return wk_fail(-(int)e, "wk_fit_step: %s", cudaGetErrorString(e));
+      return wk_check_launch("wk_fit_step");
+    }
+  }
   bool use_tma = d->kernel == WK_KERNEL_TMA;
   if (d->kernel == WK_KERNEL_TMA || (d->kernel == WK_KERNEL_AUTO && big)) {
     FitParams<T> p0 = make_params<T>(d, par);

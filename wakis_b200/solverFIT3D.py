@@ -160,6 +160,7 @@ class SolverFIT3D(RoutinesMixin):
                           "itAx", "itAy", "itAz")}
         self._zc = torch.as_tensor(self.z, dtype=torch.float64, device=dev)
         self._status = torch.zeros(1, dtype=torch.int32, device=dev)
+        self._sync = torch.zeros(_native.WK_SYNC_WORDS, dtype=torch.int32, device=dev)
         sd = self.state_dtype
         self.E = StateField(self, self._E, self.Nx, self.Ny, self.Nz, sd)
         self.H = StateField(self, self._H, self.Nx, self.Ny, self.Nz, sd)
@@ -189,6 +190,7 @@ class SolverFIT3D(RoutinesMixin):
         d.use_conductivity = int(self.use_conductivity)
         d.zc = self._zc.data_ptr()
         d.status = self._status.data_ptr()
+        d.sync = self._sync.data_ptr()
         self._desc = d
         self.kernel = "auto"
         # (tile rows, planes per block), 0 = automatic: the rows pick the
