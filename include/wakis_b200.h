@@ -115,8 +115,8 @@ typedef struct wk_fit_desc {
    * tile_planes (0 = automatic) sets the planes per block of the TMA kernel
    * and the planes per thread of the two-pass kernels.  tile_rows sets the
    * tile shape of the TMA kernels and of the batched launches: 8 for 64x8
-   * tiles, 16 for 32x16 tiles, 0 for the faster on B200 (64x8 in FP64 and
-   * FP32; in WK_F32C 32x16 on planes of 256x256 cells or more, else 64x8;
+   * tiles, 16 for 32x16 tiles, 0 for the faster on B200 (FP64 and FP32: the
+   * one that covers the plane with fewer lanes, 64x8 when equal; in WK_F32C 32x16 on planes of 256x256 cells or more, else 64x8;
    * 32x16 in the batched launches).                                        */
   int kernel;
   int tile_rows, tile_planes;
@@ -174,9 +174,11 @@ typedef struct wk_fit_desc {
 
 #define WK_SYNC_WORDS 96
 
-#define WK_KERNEL_AUTO 0   /* WK_KERNEL_TMA when its conditions hold, else
-                              WK_KERNEL_TWOPASS when Nx, Ny, Nz >= 5, else
-                              WK_KERNEL_CELL                                */
+#define WK_KERNEL_AUTO 0   /* the fastest on B200: the TMA kernel (also on
+                              rows that are no multiple of 16 bytes), all
+                              steps of a call in one launch on small grids
+                              (sync), WK_KERNEL_TWOPASS when Nx, Ny, Nz >= 5,
+                              else WK_KERNEL_CELL                           */
 #define WK_KERNEL_CELL 1   /* one thread per cell, general row code, H of
                               the backward neighbours recomputed            */
 #define WK_KERNEL_TWOPASS 4 /* H pass then E pass, each an interior launch

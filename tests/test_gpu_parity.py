@@ -218,6 +218,43 @@ def test_schedules_equal_cell_kernel_with_beam_and_capture(kernel, tile):
     assert torch.equal(ha, hb)
 
 
+@pytest.mark.parametrize("dtype,precision_shape", [
+    (np.float64, (133, 67, 47)), (np.float64, (65, 77, 81)), (np.float32, (131, 67, 47)),
+    (np.float32, (70, 77, 81)), (np.float32, (33, 129, 97))])
+@pytest.mark.parametrize("rows", [8, 16])
+@pytest.mark.parametrize("bcs", [(["pec"] * 3, ["pec"] * 3),
+                                 (["pec", "pec", "abc"], ["pec", "pec", "abc"]),
+                                 (["periodic", "periodic", "pec"], ["periodic", "periodic", "pml"]),
+                                 (["pmc", "pec", "abc"], ["pec", "pec", "pec"])])
+def test_tma_on_row_groups_equals_twopass(dtype, precision_shape, rows, bcs):
+    """Grids whose rows are no multiple of 16 bytes: the TMA kernel on groups
+    of two or four rows (one step per launch) equals the two-pass schedule
+    value for value, from random fields on every entry (unclean faces, the
+    rows of the last partial group), with the beam and the capture."""
+    import wakis_b200 as wb
+    from wakis_b200.sources import Beam
+    sol = []
+    for kernel in ("auto", "twopass"):
+        g = wb.GridFIT3D(-0.03, 0.031, -0.02, 0.022, -0.04, 0.043, *precision_shape, verbose=0)
+        m = np.zeros(precision_shape, bool)
+        m[5:29, 7:40, 9:30] = True
+        g.add_solid("a", m, [4.0, 1.0, 10.0])
+        s = wb.SolverFIT3D(g, bc_low=bcs[0], bc_high=bcs[1], dtype=dtype, bg=[1.0, 1.0],
+                           use_stl=True, use_sibc=False, verbose=0)
+        s.kernel, s.tile, s.steps_per_launch = kernel, (rows, 0), 1
+        rng = np.random.default_rng(7)
+        s._first_step()
+        s.E.fromarray(300 * rng.standard_normal(3 * s.N))
+        s.H.fromarray(rng.standard_normal(3 * s.N))
+        h = torch.zeros((9, s.Nz, 5), dtype=s._cap_dtype, device="cuda")
+        s._advance(5, 0, beam=Beam(q=1e-9, sigmaz=0.005).params(s), capture=(h, 20, 20, 3, 3))
+        s.check_status()
+        sol.append((s, h))
+    (a, ha), (b, hb) = sol
+    assert torch.equal(a.E.array, b.E.array) and torch.equal(a.H.array, b.H.array)
+    assert torch.equal(ha, hb)
+
+
 @pytest.mark.parametrize("shape", [(7, 5, 9), (16, 13, 40), (67, 9, 23), (33, 41, 57)])
 @pytest.mark.parametrize("idx", VALID)
 def test_many_steps_per_launch_equal_cell_kernel(idx, shape):

@@ -232,6 +232,12 @@ cudaError_t launch_shell_pair(const FitParams<T>& p, long long step, cudaStream_
 // TMA-staged fused step (fit_tma.cu): interior tiles + shell launches.
 template <typename T>
 bool tma_supported(const FitParams<T>& p);
+// Row and component pitch of 16 bytes.
+template <typename T>
+bool tma_pitch(const FitParams<T>& p);
+// Faster than the two-pass schedule on this grid.
+template <typename T>
+bool tma_preferred(const FitParams<T>& p);
 template <typename T>
 cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
                        int rows);

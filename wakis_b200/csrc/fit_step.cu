@@ -115,9 +115,9 @@ int run_fused(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_t s
     FitParams<T> p0 = make_params<T>(d, par);
     FitParams<T> p1 = make_params<T>(d, par ^ 1);
     const bool ok = tma_supported<T>(p0) && tma_supported<T>(p1);
-    if (d->kernel == WK_KERNEL_TMA && !ok)
+    if (d->kernel == WK_KERNEL_TMA && !(ok && tma_pitch<T>(p0)))
       return wk_fail(WK_E_SHAPE, "wk_fit_step: TMA kernel needs a 16-byte row pitch, dims >= 5");
-    use_tma = ok;
+    use_tma = ok && (d->kernel == WK_KERNEL_TMA || tma_preferred<T>(p0));
   }
   if (use_tma) {
     int s = 0;

@@ -74,37 +74,70 @@ struct TShape {
 template <typename T, int TW>
 constexpr int h_box_x() { return sizeof(T) == 8 ? TW + 2 : TW + 4; }
 
+// One map per component, or (row groups) e[0] and h[0] over all rows.
 struct TmaMaps {
   CUtensorMap e[3];
   CUtensorMap h[3];
 };
 
+// Row groups (GRP): a row pitch that is no multiple of 16 bytes becomes one when
+// kGroup = 2 or 4 rows are taken together, so the rows of a field (all three
+// components, in flat order) form a 2-D tensor of `group` Nx wide super-rows,
+// and a tile's rows of each residue (flat row mod group) are one box of it.
+// Per component a slot holds `group` boxes of grp_rows() rows; a row starts at ext column 0 rounded down to 16 bytes.  The offset of ext
+// column 0 of every (component, ext row) is tabulated per slot by warp 9 when
+// it issues the boxes (the residues of a plane's rows change with the plane).
+// The rows past the last whole super-row are copied by hand.
+// Measured on B200 against the two-pass schedule (us a step): 149x131x301 FP64
+// with open ends 288 / 165, 223x177x200 FP64 324 / 195, 81x77x160 FP64 closed
+// 68 / 35, 101x99x203 FP32 79 / 60, 223x177x400 FP32 454 / 320; one bulk copy
+// per row instead of boxes of rows took 239 and 417 us on the first and last.
+constexpr int grp_rows(int rows, int group) { return (rows + group - 1) / group; }
+template <typename T>
+constexpr int kGroupMax = sizeof(T) == 8 ? 2 : 4;
+template <typename T>
+constexpr int kRowElems = 16 / (int)sizeof(T);
+
 // Box geometry.  The interior variant loads E on x in [i0-2, i0+TX+2) and
 // H on [i0-2, i0+TX) (i0 = 2 + TX bx); the full-domain variant (FULL, tiles
 // from i0 = TX bx) starts both boxes at i0-4 so that the x offset stays
 // 16-byte aligned for float and double: E TX+8 wide, H TX+4 wide.
-template <typename T, bool FULL, int TW = 64>
+template <typename T, bool FULL, bool GRP, int TW = 64>
 struct TmaGeom {
   using S = TShape<TW>;
-  static constexpr int ebx = FULL ? S::TX + 8 : S::BX;            // E box width
-  static constexpr int hbx = FULL ? S::TX + 4 : h_box_x<T, TW>();  // H box width
-  static constexpr int xo = FULL ? 3 : 1;                          // box x of ext column 0
+  static constexpr int row = (S::TX + 2 + 2 * (kRowElems<T> - 1)) / kRowElems<T> * kRowElems<T>;
+  static constexpr int ebx = GRP ? row : (FULL ? S::TX + 8 : S::BX);             // E box width
+  static constexpr int hbx = GRP ? row : (FULL ? S::TX + 4 : h_box_x<T, TW>());  // H box width
+  static constexpr int xo = GRP ? 0 : (FULL ? 3 : 1);              // box x of ext column 0
   static constexpr int xs_off = FULL ? 4 : 2;                      // box start = i0 - xs_off
+  // GRP: bytes from one residue's box to the next (128-byte aligned), of a
+  // component in a slot
+  __host__ __device__ static constexpr int box_bytes(int rows, int group) {
+    return round128(grp_rows(rows, group) * row * (int)sizeof(T));
+  }
+  static constexpr int grp_bytes(int rows) {
+    const int two = 2 * box_bytes(rows, 2), four = 4 * box_bytes(rows, 4);
+    return kGroupMax<T> == 4 && four > two ? four : two;
+  }
 };
 
-template <typename T, bool FULL, int TW = 64>
+template <typename T, bool FULL, bool GRP, int TW = 64>
 struct TmaLayout {
   using S = TShape<TW>;
-  using G = TmaGeom<T, FULL, TW>;
-  static constexpr int eslot = round128(G::ebx * S::BY * (int)sizeof(T));        // per comp
-  static constexpr int hslot = round128(G::hbx * S::HBY * (int)sizeof(T));
+  using G = TmaGeom<T, FULL, GRP, TW>;
+  // bytes of a slot per component
+  static constexpr int eslot = GRP ? G::grp_bytes(S::BY) : round128(G::ebx * S::BY * (int)sizeof(T));
+  static constexpr int hslot = GRP ? G::grp_bytes(S::HBY) : round128(G::hbx * S::HBY * (int)sizeof(T));
   static constexpr int e_off = 0;
   static constexpr int h_off = e_off + kES * 3 * eslot;
   static constexpr int hs_off = h_off + kHS * 3 * hslot;
   static constexpr int row_off = hs_off + round128(3 * S::Ext * (int)sizeof(T));
   static constexpr int l_off = row_off + round128(3 * S::Row * (int)sizeof(T));
   static constexpr int mat_off = l_off + round128(S::Lvals * (int)sizeof(T));
-  static constexpr int bar_off = mat_off + round128(9 * kMatSmem * (int)sizeof(T));
+  // row offsets: [kES][3][BY] of E, then [kHS][3][HBY] of H
+  static constexpr int tab_off = mat_off + round128(9 * kMatSmem * (int)sizeof(T));
+  static constexpr int tab = GRP ? round128((kES * 3 * S::BY + kHS * 3 * S::HBY) * 4) : 0;
+  static constexpr int bar_off = tab_off + tab;
   static constexpr int bytes = bar_off + (kES + kHS) * 8 + 128;   // + base alignment
 };
 
@@ -148,15 +181,16 @@ __device__ __forceinline__ RowEntry<T> row_entry(const FitParams<T>& p, int r, i
 // 2 <= k <= Nz-3 (no z face is involved there), and the shell launches
 // cover only the planes k in {0, 1, Nz-2, Nz-1}.  Warps with no cell on or
 // next to a face take the unmasked rows.
-template <typename T, bool SM, int JM, int MODE, bool DESC, int TW>
+// GRP: row groups (see TmaMaps); lg = log2 of the rows per group.
+template <typename T, bool SM, int JM, int MODE, bool DESC, bool GRP, int TW>
 __global__ void __launch_bounds__(kTmaThreads, sizeof(T) == 8 ? 2 : 3)
-k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int KC) {
+k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int KC, int lg) {
   constexpr bool FULL = MODE != 0;     // tiles cover x and y entirely
   constexpr bool ZFULL = MODE == 1;    // ... and every plane
   step = step_index(p, step);
   using S = TShape<TW>;
-  using Lay = TmaLayout<T, (MODE != 0), TW>;
-  using G = TmaGeom<T, (MODE != 0), TW>;
+  using Lay = TmaLayout<T, (MODE != 0), GRP, TW>;
+  using G = TmaGeom<T, (MODE != 0), GRP, TW>;
   constexpr int HBX = G::hbx;
   constexpr int EBX = G::ebx;
   constexpr int XO = G::xo;
@@ -173,6 +207,8 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
   T* stLx = sLy + S::TY + 1;                         // tLx(i0..i0+TX-1)
   T* stLy = stLx + S::TX;                            // tLy(j0..j0+TY-1)
   T* smat = reinterpret_cast<T*>(sm + Lay::mat_off);
+  int* etab = reinterpret_cast<int*>(sm + Lay::tab_off);           // [kES][3][BY] (GRP)
+  int* htab = etab + kES * 3 * S::BY;                              // [kHS][3][HBY]
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + Lay::bar_off);  // E slots, then H slots
 
   const int Nx = p.Nx, Ny = p.Ny;
@@ -186,15 +222,47 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
   // warp 9, which owns no cell
   const bool prod = tid == kTmaThreads - 1;
   const int pstart = k0 - 1;
-  const uint32_t e_bytes = (uint32_t)(3 * EBX * S::BY * sizeof(T));
-  const uint32_t h_bytes = (uint32_t)(3 * HBX * S::HBY * sizeof(T));
+  // GRP: warp 9 issues E and warp 8 H (boxes and tables), else the producer
+  // lane alone
+  const bool issue_we = GRP ? tid >= kTmaThreads - 32 : prod;
+  const bool issue_wh = GRP ? tid >= kTmaThreads - 64 && tid < kTmaThreads - 32 : prod;
+  const int grp = 1 << lg;
+  const uint32_t e_bytes =
+      (uint32_t)(3 * EBX * (GRP ? grp_rows(S::BY, grp) << lg : S::BY) * sizeof(T));
+  const uint32_t h_bytes =
+      (uint32_t)(3 * HBX * (GRP ? grp_rows(S::HBY, grp) << lg : S::HBY) * sizeof(T));
 
   if (prod) {
     for (int s = 0; s < kES + kHS; s++) mbar_init(&bar[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // GRP: the boxes of plane q (rows j0 - 1 + y of all components) and the
+  // offsets of their rows
+  auto issue_group = [&](int q, T* slot, int size, int rows, int* tab, const CUtensorMap* map,
+                         uint64_t* b) {
+    const int lane = tid & 31, box = G::box_bytes(rows, grp) / (int)sizeof(T);
+    const int r0 = q * Ny + ys, comp = Ny * Nz;
+    for (int t = lane; t < 3 * rows; t += 32) {
+      const int d = t / rows, r = d * comp + r0 + (t - d * rows), c = r & (grp - 1);
+      const int first = (d * comp + r0 - c + grp - 1) >> lg;     // first super-row of residue c
+      const int x = c * Nx + i0 - 1;
+      tab[t] = d * size + c * box + ((r >> lg) - first) * EBX + (x & (kRowElems<T> - 1));
+    }
+    if (lane < 3 * grp) {
+      const int d = lane >> lg, c = lane & (grp - 1);
+      const int first = (d * comp + r0 - c + grp - 1) >> lg;
+      tma_load_2d(slot + d * size + c * box, map, (c * Nx + i0 - 1) & ~(kRowElems<T> - 1),
+                  first, b);
+    }
+  };
   auto issue_e = [&](int q) {
     const int slot = (q - pstart) % kES;
+    if (GRP) {
+      if ((tid & 31) == 31) mbar_expect_tx(&bar[slot], e_bytes);
+      __syncwarp();
+      issue_group(q, Eb + slot * 3 * SE, SE, S::BY, etab + slot * 3 * S::BY, &maps.e[0], &bar[slot]);
+      return;
+    }
     mbar_expect_tx(&bar[slot], e_bytes);
 #pragma unroll
     for (int d = 0; d < 3; d++)
@@ -202,6 +270,13 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
   };
   auto issue_h = [&](int q) {
     const int slot = (q - pstart) % kHS;
+    if (GRP) {
+      if ((tid & 31) == 31) mbar_expect_tx(&bar[kES + slot], h_bytes);
+      __syncwarp();
+      issue_group(q, Hb + slot * 3 * SH, SH, S::HBY, htab + slot * 3 * S::HBY, &maps.h[0],
+                  &bar[kES + slot]);
+      return;
+    }
     mbar_expect_tx(&bar[kES + slot], h_bytes);
 #pragma unroll
     for (int d = 0; d < 3; d++)
@@ -214,12 +289,26 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
     return mbar_wait(&bar[kES + (q - pstart) % kHS], (uint32_t)(((q - pstart) / kHS) & 1), lim);
   };
   // E planes pstart..k1 and H planes pstart..k1-1 are loaded, each exactly
-  // once; e_hi / h_hi (producer) track the last plane issued
-  int e_hi = pstart - 1, h_hi = pstart - 1;
-  if (prod) {
-    for (int q = pstart; q <= min(pstart + kES - 1, k1); q++) { issue_e(q); e_hi = q; }
-    for (int q = pstart; q <= min(pstart + kHS - 1, k1 - 1); q++) { issue_h(q); h_hi = q; }
-  }
+  // once
+  if (GRP) __syncthreads();            // barrier set-up before the other lanes issue
+  // GRP: rows of the last, partial super-row (the last rows of Ez, Hz on the
+  // top plane), read by warp 9 once the boxes of the slot have arrived (which
+  // leave zeros there)
+  auto patch = [&](int q, T* slot, const int* tab, int rows, int W, const T* F) {
+    const int done = 3 * Ny * Nz >> lg << lg;
+    for (int y = 0; y < rows; y++) {
+      const int r = (2 * Nz + q) * Ny + ys + y;
+      if (q != Nz - 1 || r < done || r >= 3 * Ny * Nz) continue;
+      for (int x = tid & 31; x < W; x += 32) {
+        const long long n = (long long)r * Nx + i0 - 1 + x;
+        slot[tab[2 * rows + y] + x] = n < 3 * N ? F[n] : T(0);
+      }
+    }
+  };
+  if (issue_we)
+    for (int q = pstart; q <= min(pstart + kES - 1, k1); q++) issue_e(q);
+  if (issue_wh)
+    for (int q = pstart; q <= min(pstart + kHS - 1, k1 - 1); q++) issue_h(q);
 
   // owned cells, in ext-tile coordinates (ea, eb) with the origin at
   // (i0-1, j0-1).  64x8: warps 0-7 the tile cells (lane+1, w+1) and
@@ -343,15 +432,31 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
     cp_async_wait<1>();          // this thread's row entry of plane pl
     bool got = true;
     if (prod) got = wait_e(pl, lim) && wait_e(pl + 1, lim) && wait_h(pl, lim);
+    if (GRP && issue_we && pl + 1 >= Nz - 1) {
+      // the top plane arrived as E(pl) at the start of a chunk, else as E(pl+1)
+      __syncwarp();
+      const int se2 = se == kES - 1 ? 0 : se + 1;
+      if (pl == pstart || pl + 1 == Nz - 1) {
+        if (pl == pstart) patch(pl, Eb + se * 3 * SE, etab + se * 3 * S::BY, S::BY, S::TX + 2, p.E_in);
+        patch(pl + 1, Eb + se2 * 3 * SE, etab + se2 * 3 * S::BY, S::BY, S::TX + 2, p.E_in);
+      }
+      patch(pl, Hb + sh * 3 * SH, htab + sh * 3 * S::HBY, S::HBY, S::TX + 1, p.H_in);
+    }
     ok = __syncthreads_and(got);
     if (!ok) break;
     const bool prologue = pl == pstart;
-    if (prod && !prologue) {
-      // the slots of E(pl-1) and H(pl-1) are free: every thread finished plane pl-1
+    // the slots of E(pl-1) and H(pl-1) are free: every thread finished plane
+    // pl-1.  LATE: boxes and tables are formed after the H phase, while the tile
+    // warps compute E: the float H phase is so short that it waits for warp 9
+    // (223x177x400: 320 us a step against 330), the double one is not, and the
+    // boxes then arrive late (149x131x301: 177 us against 165)
+    constexpr bool LATE = GRP && sizeof(T) == 4;
+    auto issue_next = [&]() {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      if (pl + kES - 1 <= k1) { issue_e(pl + kES - 1); e_hi = pl + kES - 1; }
-      if (pl + kHS - 1 <= k1 - 1) { issue_h(pl + kHS - 1); h_hi = pl + kHS - 1; }
-    }
+      if (issue_we && pl + kES - 1 <= k1) issue_e(pl + kES - 1);
+      if (issue_wh && pl + kHS - 1 <= k1 - 1) issue_h(pl + kHS - 1);
+    };
+    if (!LATE && (issue_we || issue_wh) && !prologue) issue_next();
     // prefetch the ids of plane pl+1
     const bool more = pl + 1 < k1;
     int idn[2] = {0, 0};
@@ -378,6 +483,20 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
     const bool zf0 = ZFULL && (pl == 0 || pl == Nz - 1), zf1 = ZFULL && pl + 1 >= Nz - 1;
     const bool masked = FULL && (warp_face || zf0 || zf1);
 
+    // GRP: offsets of the rows a cell reads (E of the row: x, y, z, of the next
+    // row: x, z, of the plane above: x, y; H of the row); on 64x8 tiles one row
+    // per thread
+    int of[10];
+    auto load_offsets = [&](int eb) {
+      const int *te = etab + se * 3 * S::BY + eb, *te1 = etab + se1 * 3 * S::BY + eb,
+                *th = htab + sh * 3 * S::HBY + eb;
+      of[0] = te[0]; of[1] = te[S::BY]; of[2] = te[2 * S::BY];
+      of[3] = te[1]; of[4] = te[2 * S::BY + 1];
+      of[5] = te1[0]; of[6] = te1[S::BY];
+      of[7] = th[0]; of[8] = th[S::HBY]; of[9] = th[2 * S::HBY];
+    };
+    if (GRP && S::DY == 0) load_offsets(eb0);
+
     // new H of the owned cells (tile cells only in the prologue; FULL: no H
     // below plane 0, the ext cells outside the grid hold 0)
     T hxn[2], hyn[2];
@@ -393,20 +512,33 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
       }
       if (!hval[r] || (prologue && !tile_cell) || (ZFULL && pl < 0)) continue;
       const int ea = ea0 + S::DX * r, eb = eb0 + S::DY * r;
-      const int bi = eb * EBX + ea + XO;
-      const int hb = eb * HBX + ea + XO;
       const T* m0 = mat + 9 * id[r];
       const T R0 = mul(R[eb], m0[3]);
       const T R1 = mul(R[S::RY + ea], m0[4]);
       const T R2 = mul(iAz[r], m0[5]);
-      T hx = Hk[hb], hy = Hk[SH + hb], hz = Hk[2 * SH + hb];
-      T ex0 = Ek[bi], ey0 = Ek[SE + bi], ez0 = Ek[2 * SE + bi];
-      T ey1 = Ek[SE + bi + 1], ez1 = Ek[2 * SE + bi + 1];
-      T ex2 = Ek[bi + EBX], ez2 = Ek[2 * SE + bi + EBX];
-      T ex3 = Ek1[bi], ey3 = Ek1[SE + bi];
-      if (masked && !p.faces_clean) {
+      T hx, hy, hz, ex0, ey0, ez0, ey1, ez1, ex2, ez2, ex3, ey3;
+      if (GRP) {
+        if (S::DY != 0) load_offsets(eb);
+        const T* const Ha = Hk + ea;
+        const T* const Ea = Ek + ea;
+        const T* const E1 = Ek1 + ea;
+        hx = Ha[of[7]], hy = Ha[of[8]], hz = Ha[of[9]];
+        ex0 = Ea[of[0]], ey0 = Ea[of[1]], ez0 = Ea[of[2]];
+        ey1 = Ea[of[1] + 1], ez1 = Ea[of[2] + 1];
+        ex2 = Ea[of[3]], ez2 = Ea[of[4]];
+        ex3 = E1[of[5]], ey3 = E1[of[6]];
+      } else {
+        const int bi = eb * EBX + ea + XO, hb = eb * HBX + ea + XO;
+        hx = Hk[hb], hy = Hk[SH + hb], hz = Hk[2 * SH + hb];
+        ex0 = Ek[bi], ey0 = Ek[SE + bi], ez0 = Ek[2 * SE + bi];
+        ey1 = Ek[SE + bi + 1], ez1 = Ek[2 * SE + bi + 1];
+        ex2 = Ek[bi + EBX], ez2 = Ek[2 * SE + bi + EBX];
+        ex3 = Ek1[bi], ey3 = Ek1[SE + bi];
+      }
+      if (masked && (!p.faces_clean || (GRP && pl == Nz - 1))) {
         // E column entries tangential to a face they lie on are masked
-        // (with faces_clean those entries are +0 already)
+        // (with faces_clean those entries are +0 already; GRP: what lies past
+        // the last plane is not)
         const T z = T(0);
         ex0 = (yf0[r] || zf0) ? z : ex0;
         ey0 = (xf0[r] || zf0) ? z : ey0;
@@ -435,6 +567,7 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
 
     // warps 8 and 9 own no E row: the row slot of plane pl-1 is free (every
     // thread passed the top barrier of plane pl), stage the row of pl+2
+    if (LATE && warp >= 8 && !prologue) issue_next();
     if (warp >= 8) stage_row(pl + 2, se == 0 ? kES - 1 : se - 1);
     if (!prologue) {
       const T tLz = R[S::RL + 1];
@@ -460,7 +593,15 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
           if (xf0[r] || zf0) curl[1] = T(0);
           if (xf0[r] || yf0[r]) curl[2] = T(0);
         }
-        const T eold[3] = {Ek[bi], Ek[SE + bi], Ek[2 * SE + bi]};
+        T eold[3];
+        if (GRP) {
+          const int* te = etab + se * 3 * S::BY + b + 1;
+#pragma unroll
+          for (int d = 0; d < 3; d++) eold[d] = Ek[te[d * S::BY] + a + 1];
+        } else {
+#pragma unroll
+          for (int d = 0; d < 3; d++) eold[d] = Ek[d * SE + bi];
+        }
         Cell cc;
         cc.i = ci[r]; cc.j = cj[r]; cc.k = pl;
         if (cell_bits & (1 << r)) capture(p, cc, n, step, eold[2]);
@@ -496,8 +637,8 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
     // loads this block issued, then return
     if (prod) {
       if (p.status) atomicExch(p.status, 1);
-      for (int q = pl; q <= e_hi; q++) wait_e(q, kWaitNs);
-      for (int q = pl; q <= h_hi; q++) wait_h(q, kWaitNs);
+      for (int q = pl; q <= min(max(pl + 1, pstart + kES - 1), k1); q++) wait_e(q, kWaitNs);
+      for (int q = pl; q <= min(max(pl, pstart + kHS - 1), k1 - 1); q++) wait_h(q, kWaitNs);
     }
     __syncthreads();
   }
@@ -519,44 +660,37 @@ static bool encode_comp(CUtensorMap* map, const T* base, int Nx, int Ny, int Nz,
   return r == CUDA_SUCCESS;
 }
 
-// True when the TMA kernel can run this grid: 16-byte strides and bases
-// (Nx*sizeof(T) multiple of 16 and N even), dims >= 5, fewer than 2^31
-// cells, the driver entry point present.
+// All rows of a field as `group` Nx wide super-rows.
 template <typename T>
-bool tma_supported(const FitParams<T>& p) {
-  if (p.Nx < 5 || p.Ny < 5 || p.Nz < 5) return false;
-  if (p.N >= (1LL << 31)) return false;
-  if ((p.Nx * sizeof(T)) % 16 != 0 || (p.N * sizeof(T)) % 16 != 0) return false;
-  if (((uintptr_t)p.E_in % 16) || ((uintptr_t)p.H_in % 16)) return false;
-  return tma_encode_fn() != nullptr;
+static bool encode_rows(CUtensorMap* map, const T* base, const FitParams<T>& p, int group, int bx,
+                        int by) {
+  const CUtensorMapDataType dt =
+      sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  const long long rows = 3LL * p.Ny * p.Nz / group;
+  cuuint64_t gdim[2] = {(cuuint64_t)p.Nx * group, (cuuint64_t)rows};
+  cuuint64_t gstr[1] = {(cuuint64_t)p.Nx * group * sizeof(T)};
+  cuuint32_t box[2] = {(cuuint32_t)bx, (cuuint32_t)by};
+  cuuint32_t est[2] = {1, 1};
+  return tma_encode_fn()(map, dt, 2, (void*)base, gdim, gstr, box, est,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launch geometry cache per device: SM count and resident blocks per SM.
-struct TmaOcc { int sms = 0, per_sm = 0; bool attr = false; };
-static TmaOcc g_occ[2][2][3][3][2][2][64];
+// Rows per group: the fewest whose length is a multiple of 16 bytes; 1 also
+// needs the components to start on one.
+template <typename T>
+static int row_group(const FitParams<T>& p) {
+  int g = 1;
+  while ((p.Nx * g * sizeof(T)) % 16 != 0) g *= 2;
+  if (g == 1 && (p.N * sizeof(T)) % 16 != 0) g = 2;
+  return g;
+}
 
-template <typename T, bool SM, int JM, int MODE, bool DESC, int TW>
-static cudaError_t tma_occupancy(TmaOcc** out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  TmaOcc& o = g_occ[sizeof(T) == 8 ? 0 : 1][SM ? 1 : 0][JM][MODE][DESC ? 1 : 0][TW == 32][dev];
-  if (!o.attr) {
-    const int smem = TmaLayout<T, (MODE != 0), TW>::bytes;
-    e = cudaFuncSetAttribute(k_tma<T, SM, JM, MODE, DESC, TW>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.per_sm, k_tma<T, SM, JM, MODE, DESC, TW>,
-                                                      kTmaThreads, smem);
-    if (e != cudaSuccess) return e;
-    if (o.per_sm < 1) o.per_sm = 1;
-    o.attr = true;
-  }
-  *out = &o;
-  return cudaSuccess;
+// Row and component pitch of 16 bytes (what an explicit WK_KERNEL_TMA needs).
+template <typename T>
+bool tma_pitch(const FitParams<T>& p) {
+  return row_group(p) == 1;
 }
 
 // TMA mode of a grid: 1 when every face carries the PEC column mask, 2
@@ -569,19 +703,71 @@ static int tma_mode(const FitParams<T>& p) {
   return (p.pec_face[4] == 0 && p.pec_face[5] == 0) ? 1 : 2;
 }
 
-template <typename T, bool SM, int JM, int MODE, bool DESC, int TW>
+// The TMA kernel on row groups needs a shell pair after it unless every face
+// is PEC-masked; on small grids the two passes are then as fast.  Measured on
+// B200, two-pass / TMA (us a step): 33x37x65 FP64 periodic 29.0 / 29.1, open
+// ends 29.2 / 28.6, 45x45x110 FP64 periodic 43.6 / 41.4; 45x45x110 FP32 open
+// 30.4 / 32.2, 61x61x130 FP32 periodic 45.2 / 43.4, open 43.7 / 34.2.
+template <typename T>
+bool tma_preferred(const FitParams<T>& p) {
+  return row_group(p) == 1 || tma_mode(p) == 1 || p.N >= (sizeof(T) == 8 ? 100000 : 400000);
+}
+
+// True when the TMA kernel can run this grid: 16-byte aligned buffers, dims
+// >= 5, fewer than 2^31 cells, the driver entry point present.
+template <typename T>
+bool tma_supported(const FitParams<T>& p) {
+  if (p.Nx < 5 || p.Ny < 5 || p.Nz < 5) return false;
+  if (p.N >= (1LL << 31)) return false;
+  if (((uintptr_t)p.E_in % 16) || ((uintptr_t)p.H_in % 16)) return false;
+  return tma_encode_fn() != nullptr;
+}
+
+// Launch geometry cache per device: SM count and resident blocks per SM.
+struct TmaOcc { int sms = 0, per_sm = 0; bool attr = false; };
+static TmaOcc g_occ[2][2][3][3][2][2][2][64];
+
+template <typename T, bool SM, int JM, int MODE, bool DESC, bool GRP, int TW>
+static cudaError_t tma_occupancy(TmaOcc** out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  TmaOcc& o = g_occ[sizeof(T) == 8 ? 0 : 1][SM ? 1 : 0][JM][MODE][DESC ? 1 : 0][GRP ? 1 : 0][TW == 32][dev];
+  if (!o.attr) {
+    const int smem = TmaLayout<T, (MODE != 0), GRP, TW>::bytes;
+    e = cudaFuncSetAttribute(k_tma<T, SM, JM, MODE, DESC, GRP, TW>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    e = cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.per_sm, k_tma<T, SM, JM, MODE, DESC, GRP, TW>,
+                                                      kTmaThreads, smem);
+    if (e != cudaSuccess) return e;
+    if (o.per_sm < 1) o.per_sm = 1;
+    o.attr = true;
+  }
+  *out = &o;
+  return cudaSuccess;
+}
+
+template <typename T, bool SM, int JM, int MODE, bool DESC, bool GRP, int TW>
 static cudaError_t launch_tma_variant(const FitParams<T>& p, long long step, cudaStream_t st,
                                       int KC) {
   using S = TShape<TW>;
-  using G = TmaGeom<T, (MODE != 0), TW>;
-  TmaMaps maps;
-  for (int d = 0; d < 3; d++) {
+  using G = TmaGeom<T, (MODE != 0), GRP, TW>;
+  TmaMaps maps = {};
+  const int group = GRP ? row_group(p) : 1;
+  if (GRP && (!encode_rows(&maps.e[0], p.E_in, p, group, G::ebx, grp_rows(S::BY, group)) ||
+              !encode_rows(&maps.h[0], p.H_in, p, group, G::hbx, grp_rows(S::HBY, group))))
+    return cudaErrorInvalidValue;
+  for (int d = 0; d < 3 && !GRP; d++) {
     if (!encode_comp<T>(&maps.e[d], p.E_in + d * p.N, p.Nx, p.Ny, p.Nz, G::ebx, S::BY) ||
         !encode_comp<T>(&maps.h[d], p.H_in + d * p.N, p.Nx, p.Ny, p.Nz, G::hbx, S::HBY))
       return cudaErrorInvalidValue;
   }
   TmaOcc* occ = nullptr;
-  cudaError_t e = tma_occupancy<T, SM, JM, MODE, DESC, TW>(&occ);
+  cudaError_t e = tma_occupancy<T, SM, JM, MODE, DESC, GRP, TW>(&occ);
   if (e != cudaSuccess) return e;
   const int span_x = MODE ? p.Nx : p.Nx - 4, span_y = MODE ? p.Ny : p.Ny - 4;
   const int planes = MODE == 1 ? p.Nz : p.Nz - 4;
@@ -590,9 +776,9 @@ static cudaError_t launch_tma_variant(const FitParams<T>& p, long long step, cud
     KC = tma_auto_kc((long long)gx * gy, planes, (long long)occ->sms * occ->per_sm);
   const int gz = (planes + KC - 1) / KC;
   timer_begin(st);
-  k_tma<T, SM, JM, MODE, DESC, TW><<<dim3(gx, gy, gz), kTmaThreads,
-                                     TmaLayout<T, (MODE != 0), TW>::bytes, st>>>(p, maps, step,
-                                                                                 KC);
+  k_tma<T, SM, JM, MODE, DESC, GRP, TW><<<dim3(gx, gy, gz), kTmaThreads,
+                                          TmaLayout<T, (MODE != 0), GRP, TW>::bytes, st>>>(
+      p, maps, step, KC, group == 4 ? 2 : group - 1);
   timer_end(st);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -603,9 +789,25 @@ static cudaError_t launch_tma_variant(const FitParams<T>& p, long long step, cud
   return launch_shell_pair<T>(p, step, st, MODE == 2);
 }
 
+// Whether 32x16 tiles take less time than 64x8 ones: the lanes of the tiles
+// that cover the plane, times what a 32x16 tile costs more; on small grids,
+// which do not fill the SMs, 64x8 (61x61x130 FP64 18.9 / 20.3).  Measured on B200,
+// 64x8 / 32x16 (us a step): 256x256x512 FP64 576 / 585, FP32 399 / 423 (equal
+// lanes); 160x128x300 FP64 145 / 134, 149x131x301 FP64 185 / 165, 96x96x240
+// FP64 103 / 96, 150x150x300 FP32 168 / 168, 101x99x203 FP32 60 / 65,
+// 223x177x400 FP32 320 / 333.
+template <typename T>
+static bool tma_narrow(const FitParams<T>& p, bool grp) {
+  auto lanes = [&](int tx) {
+    const int ty = 512 / tx;
+    return (long long)((p.Nx + tx - 1) / tx * tx) * ((p.Ny + ty - 1) / ty * ty);
+  };
+  const double more = sizeof(T) == 8 ? 1.03 : (grp ? 1.14 : 1.07);
+  return p.N >= 600000 && more * (double)lanes(32) < (double)lanes(64);
+}
+
 // One step with the TMA kernel in the mode the faces allow (see k_tma), on
-// 64x8 tiles (rows 8 or 0, the faster on B200 at 256x256x512 in FP64 and
-// FP32) or 32x16 tiles (rows 16).
+// 64x8 tiles (rows 8), 32x16 tiles (rows 16) or the better of the two (rows 0).
 template <typename T>
 cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
                        int rows) {
@@ -613,11 +815,16 @@ cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, i
   const int jm = p.j_mode == WK_J_SIGMA_E ? 1 : (p.j_mode == WK_J_ARRAY ? 2 : 0);
   const int mode = tma_mode(p);
   const bool desc = p.h_desc != 0;
-  const bool w32 = rows == 16;
+  const bool grp = row_group(p) > 1;
+  const bool w32 = rows == 16 || (rows == 0 && tma_narrow(p, grp));
 #define WK_TMA_WIDTH(SMV, JMV, MV, DV)                                                \
   {                                                                                   \
-    if (w32) return launch_tma_variant<T, SMV, JMV, MV, DV, 32>(p, step, st, KC);     \
-    return launch_tma_variant<T, SMV, JMV, MV, DV, 64>(p, step, st, KC);              \
+    if (grp) {                                                                        \
+      if (w32) return launch_tma_variant<T, SMV, JMV, MV, DV, true, 32>(p, step, st, KC); \
+      return launch_tma_variant<T, SMV, JMV, MV, DV, true, 64>(p, step, st, KC);      \
+    }                                                                                 \
+    if (w32) return launch_tma_variant<T, SMV, JMV, MV, DV, false, 32>(p, step, st, KC); \
+    return launch_tma_variant<T, SMV, JMV, MV, DV, false, 64>(p, step, st, KC);       \
   }
 #define WK_TMA_MODES(SMV, JMV, DV)                                                    \
   {                                                                                   \
@@ -645,6 +852,10 @@ int tma_launches_per_step(const FitParams<T>& p) {
   return tma_mode(p) == 1 ? 1 : 3;
 }
 
+template bool tma_preferred<double>(const FitParams<double>&);
+template bool tma_preferred<float>(const FitParams<float>&);
+template bool tma_pitch<double>(const FitParams<double>&);
+template bool tma_pitch<float>(const FitParams<float>&);
 template int tma_launches_per_step<double>(const FitParams<double>&);
 template int tma_launches_per_step<float>(const FitParams<float>&);
 template bool tma_supported<double>(const FitParams<double>&);
