@@ -18,53 +18,160 @@
 
 namespace {
 
-template <typename H>
-__global__ void k_wake_potential(const H* __restrict__ hist, long long hist_nt, int Nzh,
-                                 const int* __restrict__ win_map, int n_win, int carry,
-                                 const double* __restrict__ z, const double* __restrict__ dz,
-                                 int nz, int k_off, const double* __restrict__ s, int ns,
-                                 const long long* __restrict__ key_order, long long nt,
-                                 double v, double zmin, double zmax, double t0, double ti,
-                                 double dt, double qnorm, int counter_moving,
-                                 double* __restrict__ WP3d) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= ns) return;
-  const double sn = s[n];
-  const double zmin_v = __ddiv_rn(zmin, v);
-  const double zmax_v = __ddiv_rn(zmax, -v);
-  double prev = 0.0;
-  for (int w = 0; w < n_win; w++) {
-    double acc = carry ? prev : 0.0;
-    const H* hw = hist + (long long)win_map[w] * Nzh * hist_nt;
-    for (int k = 0; k < nz; k++) {
-      double ts;
-      int kz;
-      double coef;
-      if (!counter_moving) {
-        ts = __dadd_rn(__dsub_rn(__dsub_rn(__ddiv_rn(__dadd_rn(z[k], sn), v), zmin_v), t0), ti);
-        kz = k + k_off;
-        coef = dz[k];
-      } else {
-        int kr = nz - 1 - k;
-        ts = __dadd_rn(__dsub_rn(__dsub_rn(__ddiv_rn(__dsub_rn(z[kr], sn), -v), zmax_v), t0), ti);
-        kz = kr + k_off;
-        coef = -dz[k];
+// History column that sample s reads for the z index k of the sum, -1 for none
+// (and the row and sign of the coefficient follow from k alone).
+struct WakeArgs {
+  int nz, k_off, ns, counter_moving, n_win, carry, Nzh;
+  long long hist_nt, nt;
+  double v, zmin_v, zmax_v, t0, ti, dt, qnorm;
+};
+__device__ __forceinline__ int wake_column(const WakeArgs& g, const double* __restrict__ z,
+                                           const long long* __restrict__ key_order, double sn,
+                                           int k) {
+  const int kr = g.counter_moving ? g.nz - 1 - k : k;
+  const double zk = __ldg(z + kr);
+  const double ts =
+      g.counter_moving
+          ? __dadd_rn(__dsub_rn(__dsub_rn(__ddiv_rn(__dsub_rn(zk, sn), -g.v), g.zmax_v), g.t0), g.ti)
+          : __dadd_rn(__dsub_rn(__dsub_rn(__ddiv_rn(__dadd_rn(zk, sn), g.v), g.zmin_v), g.t0), g.ti);
+  long long it = (long long)__ddiv_rn(ts, g.dt);   // truncation toward zero, as int()
+  if (it >= g.nt) return -1;
+  if (it < 0) it += g.nt;                          // negative index wraps as in numpy
+  if (it < 0) return -1;
+  const long long t = __ldg(key_order + it);
+  return t >= 0 && t < g.hist_nt ? (int)t : -1;    // -1: no such history column
+}
+
+// One block per 32 samples.  The sum over z is sequential, window after window
+// (each starts from the one before), so the adds of a sample form one chain of
+// n_win nz terms: warp 8 runs the chains of the block's samples, one per lane,
+// and warps 0 to 7 form the terms, kWakeChunk at a time into one of two
+// shared-memory buffers, the history entries of a chunk (consecutive columns
+// of a row for the lanes of a warp) being read while the chunk before is
+// formed.  A term that does not exist is -0, which leaves any sum as it is.
+// The columns, two divisions each, are formed once per (sample, z) and kept in
+// shared memory for the other windows when they fit (COLS).
+// Bound by the chain and the history's read.  On B200, 9 windows of nz = 400,
+// ns = 11700, FP64: 272 us (345 MB), nz = 120, ns = 4700 55 us; 2632 with one thread per sample
+// that formed the column of every term and waited for its entry, 1158 with one
+// warp per block doing both parts; 4 terms per warp and chunk 257 and 85 us.
+constexpr int kWakeProd = 8, kWakeEach = 2, kWakeChunk = kWakeProd * kWakeEach;
+template <typename H, bool COLS>
+__global__ void __launch_bounds__((kWakeProd + 1) * 32)
+k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
+                 const double* __restrict__ z, const double* __restrict__ dz,
+                 const double* __restrict__ s, const long long* __restrict__ key_order,
+                 WakeArgs g, double* __restrict__ WP3d) {
+  extern __shared__ __align__(16) unsigned char wake_smem[];
+  double* term = reinterpret_cast<double*>(wake_smem);              // [2][kWakeChunk][32]
+  int* cols = reinterpret_cast<int*>(term + 2 * kWakeChunk * 32);   // [nz][32] (COLS)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = blockIdx.x * 32 + lane;
+  const bool on = n < g.ns;
+  const int terms = g.n_win * g.nz;
+  const int chunks = (terms + kWakeChunk - 1) / kWakeChunk;
+  if (warp < kWakeProd) {
+    const double sn = s[on ? n : g.ns - 1];
+    // entry and coefficient of term q (window q / nz, z index q % nz): the
+    // columns of window 0 are formed here, the others find them in `cols`
+    // (written three chunks before at least)
+    struct Terms {
+      double coef[kWakeEach];
+      H entry[kWakeEach];
+      bool have[kWakeEach];
+    };
+    auto read = [&](int chunk, Terms& v) {
+      const int q0 = chunk * kWakeChunk + warp * kWakeEach;
+      int w = q0 / g.nz, k = q0 - w * g.nz;
+#pragma unroll
+      for (int u = 0; u < kWakeEach; u++) {
+        v.have[u] = false;
+        if (q0 + u < terms) {
+          const int t = COLS && w > 0 ? cols[k * 32 + lane]
+                                      : (on ? wake_column(g, z, key_order, sn, k) : -1);
+          if (COLS && w == 0) cols[k * 32 + lane] = t;
+          const int kz = (g.counter_moving ? g.nz - 1 - k : k) + g.k_off;
+          const double c = __ldg(dz + k);
+          v.coef[u] = g.counter_moving ? -c : c;
+          v.have[u] = t >= 0;
+          v.entry[u] = v.have[u]
+                           ? hist[((long long)__ldg(win_map + w) * g.Nzh + kz) * g.hist_nt + t]
+                           : H(0);
+        }
+        if (++k == g.nz) { k = 0; w++; }
       }
-      double q = __ddiv_rn(ts, dt);
-      long long it = (long long)q;   // truncation toward zero, as int()
-      if (it < nt) {
-        if (it < 0) it += nt;          // negative index wraps as in numpy
-        if (it < 0) continue;
-        long long t = key_order[it];
-        if (t < 0 || t >= hist_nt) continue;   // no such history column
-        double e = (double)hw[(long long)kz * hist_nt + t];
-        acc = __dadd_rn(acc, __dmul_rn(e, coef));
+    };
+    auto put = [&](int chunk, const Terms& v) {
+      double* out = term + (chunk & 1) * kWakeChunk * 32 + warp * kWakeEach * 32 + lane;
+#pragma unroll
+      for (int u = 0; u < kWakeEach; u++)
+        out[u * 32] = v.have[u] ? __dmul_rn((double)v.entry[u], v.coef[u]) : -0.0;
+      __syncthreads();                       // the chunk is formed, the one before summed
+    };
+    // the entries of two chunks are on their way while a third is formed
+    Terms va, vb;
+    read(0, va);
+    read(1, vb);
+    for (int c = 0; c < chunks; c += 2) {
+      put(c, va);
+      read(c + 2, va);
+      if (c + 1 < chunks) {
+        put(c + 1, vb);
+        read(c + 3, vb);
       }
     }
-    acc = __ddiv_rn(acc, qnorm);
-    WP3d[(long long)w * ns + n] = acc;
-    prev = acc;
+  } else {
+    double acc = 0.0;
+    int w = 0, k = 0;
+    for (int c = 0; c < chunks; c++) {
+      __syncthreads();
+      const double* in = term + (c & 1) * kWakeChunk * 32 + lane;
+      if (k + kWakeChunk < g.nz) {           // no window ends in this chunk
+        double v[kWakeChunk];
+#pragma unroll
+        for (int u = 0; u < kWakeChunk; u++) v[u] = in[u * 32];
+#pragma unroll
+        for (int u = 0; u < kWakeChunk; u++) acc = __dadd_rn(acc, v[u]);
+        k += kWakeChunk;
+      } else {
+#pragma unroll 1
+        for (int u = 0; u < kWakeChunk && c * kWakeChunk + u < terms; u++) {
+          acc = __dadd_rn(acc, in[u * 32]);
+          if (++k == g.nz) {
+            acc = __ddiv_rn(acc, g.qnorm);
+            if (on) WP3d[(long long)w * g.ns + n] = acc;
+            if (!g.carry) acc = 0.0;
+            k = 0;
+            w++;
+          }
+        }
+      }
+    }
   }
+}
+
+// Largest nz whose columns are kept in shared memory; the least is such that a
+// column is written at least one barrier before it is read.
+constexpr int kWakeColsMax = 1024, kWakeColsMin = 4 * kWakeChunk;
+constexpr int kWakeTermBytes = 2 * kWakeChunk * 32 * 8;
+
+template <typename H>
+cudaError_t launch_wake_potential(const H* hist, const int* win_map, const double* z,
+                                  const double* dz, const double* s, const long long* key_order,
+                                  const WakeArgs& g, double* WP3d, cudaStream_t st) {
+  const int blocks = (g.ns + 31) / 32;
+  const int threads = (kWakeProd + 1) * 32;
+  if (g.nz >= kWakeColsMin && g.nz <= kWakeColsMax) {
+    cudaError_t e = cudaFuncSetAttribute(k_wake_potential<H, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kWakeTermBytes + kWakeColsMax * 128);
+    if (e != cudaSuccess) return e;
+    k_wake_potential<H, true><<<blocks, threads, kWakeTermBytes + g.nz * 128, st>>>(
+        hist, win_map, z, dz, s, key_order, g, WP3d);
+  } else {
+    k_wake_potential<H, false><<<blocks, threads, kWakeTermBytes, st>>>(hist, win_map, z, dz, s,
+                                                                        key_order, g, WP3d);
+  }
+  return cudaGetLastError();
 }
 
 // numpy's pairwise summation (blocks of <= 128 with 8 accumulators, halves
@@ -126,18 +233,123 @@ __device__ double pw_sum(const double* a, long long n) {
   }
 }
 
+// The same sums of [lo, lo + n) of four arrays by a group of 8 lanes (`mask`,
+// lane j of the group holds accumulator j), the result in all of them.
+struct Pw4 { double v[4]; };
+__device__ __forceinline__ Pw4 pw_leaf4(const double* const* a, int lo, int n, int j,
+                                        unsigned mask) {
+  Pw4 r;
+  if (n < 8) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) r.v[q] = -0.0;
+    for (int i = 0; i < n; i++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) r.v[q] = __dadd_rn(r.v[q], a[q][lo + i]);
+    return r;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) r.v[q] = a[q][lo + j];
+  int i = 8;
+  for (; i < n - (n % 8); i += 8)
+#pragma unroll
+    for (int q = 0; q < 4; q++) r.v[q] = __dadd_rn(r.v[q], a[q][lo + i + j]);
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int x = 1; x < 8; x *= 2)
+      r.v[q] = __dadd_rn(r.v[q], __shfl_xor_sync(mask, r.v[q], x));
+  for (; i < n; i++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) r.v[q] = __dadd_rn(r.v[q], a[q][lo + i]);
+  return r;
+}
+// ... of at most 128 * 2^D values, by a tree of calls.
+template <int D>
+__device__ __noinline__ Pw4 pw_tree4(const double* const* a, int lo, int n, int j, unsigned mask) {
+  if (n <= 128) return pw_leaf4(a, lo, n, j, mask);
+  Pw4 r;
+  if constexpr (D > 0) {
+    const int n2 = (int)pw_half(n);
+    const Pw4 left = pw_tree4<D - 1>(a, lo, n2, j, mask);
+    r = pw_tree4<D - 1>(a, lo + n2, n - n2, j, mask);
+#pragma unroll
+    for (int q = 0; q < 4; q++) r.v[q] = __dadd_rn(left.v[q], r.v[q]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; q++) r.v[q] = pw_sum(a[q] + lo, n);
+  }
+  return r;
+}
+
+// numpy's pairwise sums of a[q][0 .. n) by one warp (the results in lane 0):
+// the first five splits give 32 nodes (the bits of a node's number, highest
+// first, choose left or right), summed four at a time by the groups of 8 lanes,
+// one per lane afterwards, and added pair by pair; a node that is a leaf before
+// the fifth split is the one whose further bits are 0.
+__device__ __forceinline__ Pw4 pw_warp4(const double* const* a, int n, int lane) {
+  auto node = [&](int id, int& lo, int& len, int& depth) {
+    lo = 0;
+    len = n;
+    depth = 0;
+    bool there = true;
+#pragma unroll
+    for (int b = 4; b >= 0; b--) {
+      const bool right = id >> b & 1;
+      if (len > 128) {
+        const int n2 = (int)pw_half(len);
+        lo += right ? n2 : 0;
+        len = right ? len - n2 : n2;
+        depth++;
+      } else if (right) {
+        there = false;
+      }
+    }
+    return there;
+  };
+  const int grp = lane >> 3, j = lane & 7;
+  const unsigned mask = 0xffu << (8 * grp);
+  Pw4 r = {{0.0, 0.0, 0.0, 0.0}};
+  int lo, len, depth;
+  for (int it = 0; it < 8; it++) {
+    Pw4 v = {{0.0, 0.0, 0.0, 0.0}};
+    if (node(it * 4 + grp, lo, len, depth))
+      v = len <= 128 ? pw_leaf4(a, lo, len, j, mask) : pw_tree4<4>(a, lo, len, j, mask);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      // node it * 4 + g is in the lanes of group g, and wanted by lane it * 4 + g
+      const double x = __shfl_sync(0xffffffffu, v.v[q], (lane & 3) * 8);
+      if (lane >> 2 == it) r.v[q] = x;
+    }
+  }
+  node(lane, lo, len, depth);
+#pragma unroll
+  for (int b = 0; b < 5; b++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const double o = __shfl_down_sync(0xffffffffu, r.v[q], 1 << b);
+      if (depth >= 5 - b) r.v[q] = __dadd_rn(r.v[q], o);
+    }
+  return r;
+}
+
 // Positions (+1,0) (-1,0) (0,+1) (0,-1) are w = 7, 1, 5, 3 of the 3x3 block;
-// each thread forms the four prefix integrals of its s sample directly.
-__global__ void k_trans_wake(const double* __restrict__ WP3d, int ns, double ds, double dxsum,
-                             double dysum, double* __restrict__ WPx, double* __restrict__ WPy) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= ns) return;
-  double ixp = __dmul_rn(pw_sum(WP3d + 7LL * ns, n), ds);
-  double ixm = __dmul_rn(pw_sum(WP3d + 1LL * ns, n), ds);
-  double iyp = __dmul_rn(pw_sum(WP3d + 5LL * ns, n), ds);
-  double iym = __dmul_rn(pw_sum(WP3d + 3LL * ns, n), ds);
-  WPx[n] = __ddiv_rn(-__dsub_rn(ixp, ixm), dxsum);
-  WPy[n] = __ddiv_rn(-__dsub_rn(iyp, iym), dysum);
+// one warp forms the four prefix integrals of a sample.  O(ns^2) adds in
+// numpy's order.  On B200, ns = 11700: 151 us; 1052 with one thread
+// per sample, 623 with one node per lane (32 lines a load).
+constexpr int kTransWarps = 8;
+__global__ void __launch_bounds__(kTransWarps * 32)
+k_trans_wake(const double* __restrict__ WP3d, int ns, double ds, double dxsum, double dysum,
+             double* __restrict__ WPx, double* __restrict__ WPy) {
+  // the longest prefixes first
+  const int n = ns - 1 - (int)(blockIdx.x * kTransWarps + (threadIdx.x >> 5));
+  if (n < 0) return;
+  const double* const a[4] = {WP3d + 7LL * ns, WP3d + 1LL * ns, WP3d + 5LL * ns, WP3d + 3LL * ns};
+  const Pw4 r = pw_warp4(a, n, threadIdx.x & 31);
+  if ((threadIdx.x & 31) == 0) {
+    WPx[n] = __ddiv_rn(-__dsub_rn(__dmul_rn(r.v[0], ds), __dmul_rn(r.v[1], ds)), dxsum);
+    WPy[n] = __ddiv_rn(-__dsub_rn(__dmul_rn(r.v[2], ds), __dmul_rn(r.v[3], ds)), dysum);
+  }
 }
 
 // ------------------------------------------------------------- streaming --
@@ -234,6 +446,11 @@ __device__ __forceinline__ DD dd_add(DD a, DD b) {
   return dd_add(r, b.lo);
 }
 
+__device__ __forceinline__ DD dd_mul(double a, double b) {   // exact product
+  const double p = __dmul_rn(a, b);
+  return {p, __fma_rn(a, b, -p)};
+}
+
 constexpr int kScanThreads = 256;
 __device__ __forceinline__ int trans_win(int q) { return q == 0 ? 7 : (q == 1 ? 1 : (q == 2 ? 5 : 3)); }
 
@@ -299,36 +516,65 @@ __global__ void k_trans_final(const double* __restrict__ WP3d, int ns, int seg,
   }
 }
 
-// One block per (signal, bin); fixed-shape tree reduction (deterministic).
-constexpr int kDftThreads = 256;
-__global__ void k_dft_bins(const double* __restrict__ x, long long len, long long N,
-                           int nbins, double* __restrict__ out) {
-  int m = blockIdx.x;
-  int sig = blockIdx.y;
+// One block per (signal, bin).  With w = exp(-2 pi i m / N), thread t sums
+// x[t + T a] w^(T a) over a and multiplies once by w^t, so that a bin takes
+// about T + len / T exponentials instead of len; the exponentials w^(T a) come
+// from shared memory, kDftChunk at a time.  Fixed-shape tree reduction
+// (deterministic).  On B200, 984 bins of 11700 samples: 2 signals 25 us,
+// 3 signals 34 us; 127 us on average with one exponential per term.
+constexpr int kDftThreads = 256, kDftChunk = 256;
+// cos and sin of 2 pi m n / N, the angle brought within an eighth of a turn by
+// exact integer quarter turns first (so that its rounding, relative to a small
+// angle, stays far below the functions' own).
+__device__ __forceinline__ void dft_unit(long long m, long long n, long long N, double* c,
+                                         double* s) {
+  const long long r = (m * n) % N;
+  const long long q = (4 * r + N / 2) / N;            // quarter turns, 0 to 4
+  double sn, cs;
+  sincospi(__ddiv_rn((double)(4 * r - q * N), 2.0 * (double)N), &sn, &cs);
+  const double c0 = q & 1 ? -sn : cs, s0 = q & 1 ? cs : sn;
+  *c = q & 2 ? -c0 : c0;
+  *s = q & 2 ? -s0 : s0;
+}
+__global__ void __launch_bounds__(kDftThreads)
+k_dft_bins(const double* __restrict__ x, long long len, long long N, int nbins,
+           double* __restrict__ out) {
+  const int m = blockIdx.x, sig = blockIdx.y, t = threadIdx.x;
   const double* xs = x + (long long)sig * len;
+  __shared__ double2 unit[kDftChunk];
   double re = 0.0, im = 0.0;
-  for (long long n = threadIdx.x; n < len; n += kDftThreads) {
-    long long r = ((long long)m * n) % N;
-    double sn, cs;
-    sincospi(__ddiv_rn(2.0 * (double)r, (double)N), &sn, &cs);
-    double v = xs[n];
-    re = __dadd_rn(re, __dmul_rn(v, cs));
-    im = __dsub_rn(im, __dmul_rn(v, sn));
-  }
-  __shared__ double sre[kDftThreads], sim[kDftThreads];
-  sre[threadIdx.x] = re;
-  sim[threadIdx.x] = im;
-  __syncthreads();
-  for (int w = kDftThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      sre[threadIdx.x] = __dadd_rn(sre[threadIdx.x], sre[threadIdx.x + w]);
-      sim[threadIdx.x] = __dadd_rn(sim[threadIdx.x], sim[threadIdx.x + w]);
+  const long long steps = (len + kDftThreads - 1) / kDftThreads;
+  for (long long a0 = 0; a0 < steps; a0 += kDftChunk) {
+    const int na = (int)min((long long)kDftChunk, steps - a0);
+    if (t < na) dft_unit(m, (a0 + t) * kDftThreads, N, &unit[t].x, &unit[t].y);
+    __syncthreads();
+    for (int a = 0; a < na; a++) {
+      const long long n = (a0 + a) * kDftThreads + t;
+      if (n < len) {
+        const double v = xs[n];
+        re = __fma_rn(v, unit[a].x, re);
+        im = __fma_rn(-v, unit[a].y, im);
+      }
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    out[((long long)sig * nbins + m) * 2] = sre[0];
-    out[((long long)sig * nbins + m) * 2 + 1] = sim[0];
+  // (re + i im)(c - i s) and the tree in double-double: each bin is rounded once
+  double c, s;
+  dft_unit(m, t, N, &c, &s);
+  __shared__ DD sre[kDftThreads], sim[kDftThreads];
+  sre[t] = dd_add(dd_mul(re, c), dd_mul(im, s));
+  sim[t] = dd_add(dd_mul(im, c), dd_mul(-re, s));
+  __syncthreads();
+  for (int w = kDftThreads / 2; w > 0; w >>= 1) {
+    if (t < w) {
+      sre[t] = dd_add(sre[t], sre[t + w]);
+      sim[t] = dd_add(sim[t], sim[t + w]);
+    }
+    __syncthreads();
+  }
+  if (t == 0) {
+    out[((long long)sig * nbins + m) * 2] = __dadd_rn(sre[0].hi, sre[0].lo);
+    out[((long long)sig * nbins + m) * 2 + 1] = __dadd_rn(sim[0].hi, sim[0].lo);
   }
 }
 
@@ -350,15 +596,19 @@ extern "C" int wk_wake_potential(const void* hist, int hist_dtype, long long his
                    ns, nz, n_win, nt);
   if (ns == 0) return WK_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  int threads = 128, blocks = (ns + threads - 1) / threads;
-  if (hist_dtype == WK_F64)
-    k_wake_potential<double><<<blocks, threads, 0, st>>>(
-        (const double*)hist, hist_nt, Nzh, win_map, n_win, carry, z, dz, nz, k_off, s, ns,
-        key_order, nt, v, zmin, zmax, t0, ti, dt, qnorm, counter_moving, WP3d);
-  else
-    k_wake_potential<float><<<blocks, threads, 0, st>>>(
-        (const float*)hist, hist_nt, Nzh, win_map, n_win, carry, z, dz, nz, k_off, s, ns,
-        key_order, nt, v, zmin, zmax, t0, ti, dt, qnorm, counter_moving, WP3d);
+  if (hist_nt > 0x7fffffffLL)
+    return wk_fail(WK_E_RANGE, "wk_wake_potential: history of %lld columns", hist_nt);
+  WakeArgs g;
+  g.nz = nz; g.k_off = k_off; g.ns = ns; g.counter_moving = counter_moving;
+  g.n_win = n_win; g.carry = carry; g.Nzh = Nzh;
+  g.hist_nt = hist_nt; g.nt = nt;
+  g.v = v; g.zmin_v = zmin / v; g.zmax_v = zmax / -v; g.t0 = t0; g.ti = ti; g.dt = dt;
+  g.qnorm = qnorm;
+  const cudaError_t e =
+      hist_dtype == WK_F64
+          ? launch_wake_potential((const double*)hist, win_map, z, dz, s, key_order, g, WP3d, st)
+          : launch_wake_potential((const float*)hist, win_map, z, dz, s, key_order, g, WP3d, st);
+  if (e != cudaSuccess) return wk_fail(-(int)e, "wk_wake_potential: %s", cudaGetErrorString(e));
   return wk_check_launch("wk_wake_potential");
 }
 
@@ -368,8 +618,7 @@ extern "C" int wk_trans_wake(const double* WP3d, int ns, double ds, double dxsum
   if (ns < 0) return wk_fail(WK_E_RANGE, "wk_trans_wake: ns %d", ns);
   if (ns == 0) return WK_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  int threads = 128, blocks = (ns + threads - 1) / threads;
-  k_trans_wake<<<blocks, threads, 0, st>>>(WP3d, ns, ds, dxsum, dysum, WPx, WPy);
+  k_trans_wake<<<(ns + kTransWarps - 1) / kTransWarps, kTransWarps * 32, 0, st>>>(WP3d, ns, ds, dxsum, dysum, WPx, WPy);
   return wk_check_launch("wk_trans_wake");
 }
 

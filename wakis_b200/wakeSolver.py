@@ -179,7 +179,9 @@ class WakeSolver:
         dev = self._hist.device
         f64 = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64), device=dev)
         zt, dzt, st = f64(z), f64(self.dz), f64(s)
-        order = torch.as_tensor(self._key_order(n_keys), device=dev)
+        # up to 10^5 steps every key keeps its place
+        order = (torch.arange(n_keys, dtype=torch.int64, device=dev) if n_keys <= 100000
+                 else torch.as_tensor(self._key_order(n_keys), device=dev))
         win = torch.arange(n_win, dtype=torch.int32, device=dev)
         WP3d = torch.empty((n_win, len(s)), dtype=torch.float64, device=dev)
         hdt = _native.WK_F64 if self._hist.dtype == torch.float64 else _native.WK_F32
