@@ -396,6 +396,14 @@ int wk_zero_ghosts(const wk_fit_desc* d, void* stream);
 int wk_fit_step(const wk_fit_desc* d, int n_steps, long long step0, void* stream);
 
 /*
+ * 1 when a wk_fit_step call of n_steps steps on this descriptor runs them all
+ * in one launch (a small grid with `sync` words and the automatic kernel), 0
+ * when not, or when the descriptor is not valid.  No counterpart in the
+ * reference.
+ */
+int wk_fit_one_launch(const wk_fit_desc* d, int n_steps);
+
+/*
  * Same update with the two half-steps as separate in-place kernels (H pass,
  * then E pass); the state stays in E[par], H[par].  Reference schedule used
  * to cross-check the fused kernel of wk_fit_step.

@@ -296,6 +296,46 @@ def test_many_steps_per_launch_equal_cell_kernel(idx, shape):
     assert np.abs(a.E.numpy()).max() > 0
 
 
+@pytest.mark.parametrize("shape,z", [((16, 20, 33), "abc"), ((24, 16, 40), "pec"), ((52, 24, 9), "abc"),
+                                     ((36, 41, 57), "pml"), ((17, 21, 33), "abc"),
+                                     ((33, 16, 40), "pec"), ((51, 25, 9), "abc"),
+                                     ((30, 41, 57), "pml")])
+@pytest.mark.parametrize("clean", [True, False])
+def test_fp32c_many_steps_per_launch_equal_per_step(shape, z, clean):
+    """One launch for all steps (small grids): values, compensation words and
+    Ez history of the per-step kernels (TMA with Nx % 4 == 0, else two-pass),
+    bit for bit, with and without clean faces, with the beam, for an odd and
+    an even step count."""
+    import wakis_b200 as wb
+    from wakis_b200.sources import Beam
+    sol = []
+    for per_launch in (0, 1):
+        g = wb.GridFIT3D(-0.01, 0.012, -0.01, 0.01, -0.02, 0.021, *shape, verbose=0)
+        m = np.zeros(shape, bool)
+        m[3:9, 4:12, 2:8] = True
+        g.add_solid("a", m, [4.0, 1.0, 10.0])
+        s = wb.SolverFIT3D(g, bc_low=["pec", "pec", z], bc_high=["pec", "pec", z], n_pml=3,
+                           bg=[1.0, 1.0], use_stl=True, use_sibc=False, verbose=0,
+                           precision="fp32c")
+        s.steps_per_launch = per_launch
+        rng = np.random.default_rng(11)
+        s._first_step()
+        s.H.fromarray(rng.standard_normal(3 * s.N))
+        if not clean:
+            s.E.fromarray(300 * rng.standard_normal(3 * s.N))
+        h = torch.zeros((9, s.Nz, 13), dtype=torch.float64, device="cuda")
+        bp = Beam(q=1e-9, sigmaz=0.005).params(s)
+        s._advance(8, 0, beam=bp, capture=(h, 6, 5, 3, 3))
+        s._advance(5, 8, beam=bp, capture=(h, 6, 5, 3, 3))
+        s.check_status()
+        sol.append((s, h))
+    (a, ha), (b, hb) = sol
+    for f in ("_E", "_H", "_Ec", "_Hc"):
+        assert torch.equal(getattr(a, f)[a._par], getattr(b, f)[b._par]), f
+    assert torch.equal(ha, hb)
+    assert int(a._sync.abs().sum().item()) == 0
+
+
 def _wake_errors(a, b):
     return {n: rel_err(getattr(a, n), getattr(b, n)) for n in ("WP", "WPx", "WPy", "Z", "Zx")}
 

@@ -67,6 +67,7 @@ _SIGS = {
     "wk_last_error": (ctypes.c_char_p, []),
     "wk_zero_ghosts": (_i, [ctypes.POINTER(FitDesc), _vp]),
     "wk_fit_step": (_i, [ctypes.POINTER(FitDesc), _i, _ll, _vp]),
+    "wk_fit_one_launch": (_i, [ctypes.POINTER(FitDesc), _i]),
     "wk_fit_step_split": (_i, [ctypes.POINTER(FitDesc), _i, _ll, _vp]),
     "wk_fit_step_timed": (_i, [ctypes.POINTER(FitDesc), _i, _ll, _vp,
                                ctypes.POINTER(ctypes.c_float), ctypes.POINTER(_i)]),

@@ -21,6 +21,10 @@ the stepping of all of them is shared:
   of the device step counter (``wk_fit_desc.step_dev``), replayed Nt/2 times;
   the autotuner picks the planes per block of each distinct grid.
 
+* ``launch="loop"``: the instances one after another, all steps of each in one
+  launch, for grids that the solver runs that way (small ones: the state of a
+  grid stays in the shared memory of the SMs, and one grid fills them).
+
 Afterwards each ``WakeSolver`` integrates its own history as wakesolve does.
 """
 
@@ -149,6 +153,13 @@ def batched_ok(solvers):
     return True
 
 
+def loop_ok(solvers, n_steps):
+    """True when every solver runs n_steps steps of a call in one launch."""
+    lib = _native.lib()
+    return bool(solvers) and all(lib.wk_fit_one_launch(s._step_desc(), int(n_steps))
+                                 for s in solvers)
+
+
 def autotune_batch(solvers, candidates=BATCH_KC_CANDIDATES, forms=tuple(FORMS), steps=4,
                    policies=TILE_POLICIES):
     """Pick the launch form, the tile-shape policy and the planes per work
@@ -198,7 +209,10 @@ class BatchedWakeSolve:
     wakelength of each is set so that upstream's Nt formula gives n_steps).
     launch: "batched" (the device work list over all instances,
     wk_batch_run, for FP32-compensated instances), "graph" (replayed graph of
-    per-instance launches) or "auto" (batched when ``batched_ok``).  form:
+    per-instance launches), "loop" (one launch per instance for all its steps)
+    or "auto" (loop when ``loop_ok``: a call with 8 cavities of 40x40x96 to
+    64x64x119 cells and 900 steps took 84 ms, batched 187; else batched when
+    ``batched_ok``).  form:
     the batched launch form, "persistent", "phases" or "auto" (chosen by the
     autotuner; "persistent" without tuning).  tiles: the tile shapes of the
     batched launch, "64x8", "32x16", "fill" (per instance, the shape with
@@ -213,7 +227,7 @@ class BatchedWakeSolve:
                  launch="auto", chunk=500, form="auto", tiles="auto"):
         if n_steps < 2:
             raise ValueError("n_steps must be >= 2")
-        if launch not in ("auto", "batched", "graph"):
+        if launch not in ("auto", "batched", "graph", "loop"):
             raise ValueError(f"launch {launch!r}")
         if form not in ("auto",) + tuple(FORMS):
             raise ValueError(f"form {form!r}")
@@ -228,7 +242,11 @@ class BatchedWakeSolve:
         self.tuned = {}
         self.timing = {}
         if launch == "auto":
-            launch = "batched" if batched_ok(self.solvers) else "graph"
+            launch = ("loop" if form == "auto" and tiles == "auto" and
+                      loop_ok(self.solvers, n_steps - 1) else
+                      "batched" if batched_ok(self.solvers) else "graph")
+        elif launch == "loop" and not loop_ok(self.solvers, n_steps - 1):
+            raise ValueError("launch='loop' needs grids whose steps run in one launch")
         elif launch == "batched" and not batched_ok(self.solvers):
             raise ValueError("launch='batched' needs FP32-compensated instances with "
                              "PEC-masked x/y faces, sharing face mode, id width and J mode")
@@ -318,6 +336,20 @@ class BatchedWakeSolve:
                 s.nstep += rest
             self.tuned["launches"] = reps + (1 if tail else 0)
             self.tuned["steps_per_launch"] = chunk
+        elif self.launch == "loop":
+            states = self._setup()
+            torch.cuda.synchronize(dev)
+            t0 = time.perf_counter()
+            ev0 = torch.cuda.Event(enable_timing=True)
+            ev1 = torch.cuda.Event(enable_timing=True)
+            ev0.record()
+            for s, ws in zip(self.solvers, states):
+                s._advance(self.n_steps, 0, beam=ws["beam_params"], capture=ws["capture"])
+            ev1.record()
+            torch.cuda.synchronize(dev)
+            ms = ev0.elapsed_time(ev1)
+            wall = time.perf_counter() - t0
+            self.tuned = {"form": "loop", "launches": len(self.solvers)}
         else:
             ms, wall, states = self._run_graph(dev)
         for q, s in enumerate(self.solvers):

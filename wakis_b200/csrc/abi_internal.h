@@ -13,6 +13,10 @@ int wk_comp_step(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_
 int wk_comp_zero_ghosts(const wk_fit_desc* d, cudaStream_t st);
 int wk_comp_sigma_e(const wk_fit_desc* d, void* J, cudaStream_t st);
 
+// Whether a step call may run all its steps in one launch if the grid is small
+// enough (fit_step.cu).
+bool wk_one_launch_call(const wk_fit_desc* d, int n_steps);
+
 // Optional CUDA-event timing of the interior kernels of each step (the
 // kernels that carry the bulk of the cells), armed by wk_fit_step_timed on
 // the calling thread.  Launchers bracket each interior launch with

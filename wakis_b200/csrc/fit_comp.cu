@@ -269,6 +269,14 @@ int wk_comp_step(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_
   const bool cstencil = d->comp_stencil != 0;
   if (cstencil && d->kernel == WK_KERNEL_TMA)
     return wk_fail(WK_E_MODE, "wk_fit_step: the compensated stencil runs the two-pass kernels");
+  if (!cstencil && wk_one_launch_call(d, n_steps)) {
+    const FitParams<double> p = make_params<double>(d, par);
+    if (loop_comp_supported(p)) {
+      cudaError_t e = launch_loop_comp(d, p, n_steps, step0, st);
+      if (e != cudaSuccess) return wk_fail(-(int)e, "wk_fit_step: %s", cudaGetErrorString(e));
+      return wk_check_launch("wk_fit_step");
+    }
+  }
   if (!cstencil && (d->kernel == WK_KERNEL_AUTO || d->kernel == WK_KERNEL_TMA)) {
     tma = tma_comp_supported(d, make_params<double>(d, par));
     if (!tma && d->kernel == WK_KERNEL_TMA)

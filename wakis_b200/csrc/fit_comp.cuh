@@ -107,6 +107,13 @@ inline CompState comp_state(const wk_fit_desc* d, int par) {
   return s;
 }
 
+// New E of an FP64 row: one rounding for ieps J subtracted from the curl, one
+// for the increment added.
+__device__ __forceinline__ double comp_e_new(double dt, double ieps, double jv, double curl,
+                                             double e) {
+  return __fma_rn(dt, __fma_rn(-ieps, jv, curl), e);
+}
+
 // One shell cell of the compensated step: the state is decoded to FP64,
 // the cell takes the lean rows where they apply and the general rows
 // elsewhere, and the FP64 result is split back into (float, bf16).  H from
@@ -175,7 +182,7 @@ __device__ __forceinline__ void comp_shell_e(const FitParams<double>& p, const C
     const double eold = d == 2 ? ez_old : comp_value(st.E_in[d * N + n], st.Ec_in[d * N + n]);
     const double jv = j_in(p, d, c, n, step, eold, sigma);
     const double cu = lean ? curl[d] : e_curl_acc(p, d, c, n, ieps, hv);
-    const double enew = eold + p.dt * (cu - ieps * jv);
+    const double enew = comp_e_new(p.dt, ieps, jv, cu, eold);
     float t;
     comp_t q;
     comp_split(enew, t, q);
@@ -194,5 +201,11 @@ cudaError_t launch_tma_comp(const wk_fit_desc* d, const FitParams<double>& p, in
 // x/y faces do (shell launches over the four z-boundary planes only), else 0
 // (interior + full shell); never with PMC faces.
 int tma_comp_mode(const FitParams<double>& p);
+
+// All steps of a call in one launch, for small grids with PEC-masked x/y faces
+// and at most 64 materials (fit_loop_comp.cu); J = 0 or sigma E.
+bool loop_comp_supported(const FitParams<double>& p);
+cudaError_t launch_loop_comp(const wk_fit_desc* d, const FitParams<double>& p, int n_steps,
+                             long long step0, cudaStream_t st);
 
 }  // namespace wk

@@ -44,97 +44,9 @@
 #include "abi_internal.h"
 #include "fit_common.cuh"
 #include "fit_kernels.cuh"
-#include "fit_rows.cuh"
-#include "tma_util.cuh"
+#include "fit_loop.cuh"
 
 namespace wk {
-
-constexpr int kLoopThreads = 512;
-constexpr int kLoopMat = 64;              // materials staged in shared memory
-constexpr int kLoopSmem = 226 * 1024;
-constexpr int kLoopDim = 62;              // largest tile dimension (6-bit box coordinates)
-
-// words of wk_fit_desc.sync, one per 128 bytes
-constexpr int kSyncCount = 0, kSyncDone = 32, kSyncAbort = 64;
-
-// Tile split of a grid: block (bx, by, bz) owns [bx Nx / nbx, (bx+1) Nx / nbx)
-// and so on; the largest tile sets the shared-memory layout.
-struct LoopTiling {
-  int nbx, nby, nbz;
-  int tx, ty, tz;
-};
-
-// List entries: box coordinates (6 bits each), the nine factor bits
-// (RowBits), the three row bits and the class.
-enum RowBits { bXO = 1, bXZ = 2, bXY = 4, bYO = 8, bYZ = 16, bYX = 32, bZO = 64, bZX = 128, bZY = 256 };
-constexpr uint32_t kRegular = 0, kMasked = 1, kWrapped = 2;
-__device__ __forceinline__ uint32_t loop_entry(int a, int b, int c, int cols, int rows,
-                                               uint32_t cls) {
-  return (uint32_t)a | (uint32_t)b << 6 | (uint32_t)c << 12 | (uint32_t)cols << 18 |
-         (uint32_t)rows << 27 | cls << 30;
-}
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* a) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void red_release(unsigned* a) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a) : "memory");
-}
-
-// Thread 0: wait until `target` arrivals were counted.  False when the wait
-// ran out or another block gave up.
-__device__ __forceinline__ bool loop_wait(unsigned* sync, unsigned target, long long limit_ns) {
-  if (limit_ns < 0) return false;
-  if (ld_acquire(sync + kSyncCount) >= target) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  for (long long it = 0; it < kWaitPolls; it++) {
-    if (ld_acquire(sync + kSyncCount) >= target) return true;
-    if ((it & 63) == 63 && (ld_acquire(sync + kSyncAbort) != 0 ||
-                            (long long)(globaltimer_ns() - t0) > limit_ns))
-      return false;
-  }
-  return false;
-}
-
-// Factor bits of a cell's rows in direction DIR and whether a factor that is
-// not 0, of a row that is not masked (`rows`), takes a length other than the
-// cell's own.
-template <typename T, int DIR>
-__device__ __forceinline__ int loop_bits(const FitParams<T>& p, Cell c, int rows, bool& wrap) {
-  ColumnInv<T, DIR> ci;
-  ci.init(p, c.i, c.j);
-  const RowCols<T> f = ci.at(p, c.k);
-  auto bit = [](T v, int b) { return v != T(0) ? b : 0; };
-  int m = bit(f.xO, bXO) | bit(f.xZ, bXZ) | bit(f.xY, bXY) | bit(f.yO, bYO) | bit(f.yZ, bYZ) |
-          bit(f.yX, bYX) | bit(f.zO, bZO) | bit(f.zX, bZX) | bit(f.zY, bZY);
-  const bool wx = DIR > 0 ? c.i == p.Nx - 1 : c.i == 0;
-  wrap = (wx && (m & bYX) && (rows & 4)) || (ci.dkx && (m & bZX) && (rows & 2)) ||
-         (ci.dky && (m & bZY) && (rows & 1));
-  return m;
-}
-
-// One more entry of `key` for every thread of the warp with take: its place
-// in counters[key] (the places of a warp's entries follow each other).  Called
-// by whole warps.
-__device__ __forceinline__ int loop_place(bool take, int key, int* counters) {
-  const int lane = threadIdx.x & 31;
-  const unsigned same = __match_any_sync(0xffffffffu, take ? key : -1);
-  const int leader = __ffs(same) - 1;
-  int base = 0;
-  if (take && lane == leader) base = atomicAdd(counters + key, __popc(same));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  return base + __popc(same & ((1u << lane) - 1));
-}
-
-// Division of 0 <= n < 2^20 by d through a rounded-up reciprocal (exact:
-// the error n * 2^-32 * d / d stays below 1 / d).
-struct LoopDiv {
-  unsigned m;
-  __device__ __forceinline__ explicit LoopDiv(int d) : m(d == 1 ? 0u : 0xffffffffu / (unsigned)d + 1u) {}
-  __device__ __forceinline__ int div(int n) const { return m ? (int)__umulhi((unsigned)n, m) : n; }
-};
 
 // Shared-memory layout of the largest tile, in bytes.
 template <typename T>
@@ -246,12 +158,10 @@ k_loop(FitParams<T> p, LoopTiling tl, int n_steps, long long step0, unsigned* sy
   cp_async_commit();
   if (SMT)
     for (int q = tid; q < 9 * p.n_mat; q += TH) smat[q] = p.mat[q];
-  if (tid < 10) s_count[tid] = 0;
   __syncthreads();
-  // The three lists.  A counting pass, then a placing pass: H cells first
-  // those whose E is all the tile's own (a < tx, b < ty, c < tz, no halo),
-  // each part ordered by class (keys 0 to 5), E cells by class (6 to 8), the
-  // halo's E (9).
+  // The three lists (loop_lists): H cells first those whose E is all the tile's
+  // own (a < tx, b < ty, c < tz, no halo), each part ordered by class (keys 0
+  // to 5), E cells by class (6 to 8), the halo's E (9).
   auto h_entry = [&](int q, uint32_t& e) -> int {
     const int c = dHP.div(q), r = q - c * HP, b = dHX.div(r), a = r - b * HX;
     const int n = flat(a, b, c);
@@ -307,38 +217,8 @@ k_loop(FitParams<T> p, LoopTiling tl, int n_steps, long long step0, unsigned* sy
     return low + high > 0 && low <= 1 && high <= 1 && n >= 0 && n < N ? 9 : -1;
   };
   const int own = tx * ty * tz;
-  auto list_pass = [&](bool place) {
-    auto one = [&](int n, auto&& entry, uint32_t* list) {
-      for (int q0 = 0; q0 < n; q0 += TH) {
-        uint32_t e = 0;
-        const int key = q0 + tid < n ? entry(q0 + tid, e) : -1;
-        const int at = loop_place(key >= 0, key, s_count);
-        if (place && key >= 0) list[at] = e;
-      }
-    };
-    one(HV, h_entry, lh);
-    one(own, e_entry, le);
-    one(EV, s_entry, ls);
-  };
-  list_pass(false);
-  __syncthreads();
-  if (tid == 0) {
-    for (int g = 0; g < 3; g++) {             // counts to first places, per list
-      const int lo = g == 0 ? 0 : (g == 1 ? 6 : 9), hi = g == 0 ? 6 : (g == 1 ? 9 : 10);
-      int sum = 0;
-      for (int q = lo; q < hi; q++) {
-        const int c = s_count[q];
-        s_count[q] = sum;
-        sum += c;
-      }
-      s_len[g] = sum;
-    }
-    s_len[3] = s_count[3];                    // H cells that read the tile's own E only
-  }
-  __syncthreads();
+  loop_lists(s_count, s_len, HV, h_entry, lh, own, e_entry, le, EV, s_entry, ls);
   const int nh = s_len[0], ne = s_len[1], nsh = s_len[2], nh_own = s_len[3];
-  list_pass(true);
-  __syncthreads();
   auto id_of = [&](uint32_t e) -> IdT {
     return (IdT)load_id(p.mat_id, p.id_bytes, flat(e & 63, e >> 6 & 63, e >> 12 & 63));
   };
@@ -358,6 +238,14 @@ k_loop(FitParams<T> p, LoopTiling tl, int n_steps, long long step0, unsigned* sy
   cp_async_wait<0>();
   __syncthreads();
 
+  // cell of a box position (one before the grid: the last column of the row
+  // below, the last row of the plane below)
+  auto true_cell = [&](int a, int b, int c) {
+    Cell cc = {i0 - 1 + a, j0 - 1 + b, k0 - 1 + c};
+    if (cc.i < 0) { cc.i = Nx - 1; cc.j--; }
+    if (cc.j < 0) { cc.j += Ny; cc.k--; }
+    return cc;
+  };
   const bool desc = p.h_desc != 0;
   const T dt = p.dt;
   auto pick = [](uint32_t bits, int b, T v) { return (bits & b) ? v : T(0); };
@@ -395,11 +283,11 @@ k_loop(FitParams<T> p, LoopTiling tl, int n_steps, long long step0, unsigned* sy
              pick(w, bYO, v.L[1]), pick(w, bYZ, v.L[1]), pick(w, bYX, v.L[1]),
              pick(w, bZO, v.L[2]), pick(w, bZX, v.L[2]), pick(w, bZY, v.L[2])};
       } else {
-        const Cell cc = cell_of(flat(e & 63, e >> 6 & 63, e >> 12 & 63), Nx, Ny);
+        const Cell cc = true_cell(e & 63, e >> 6 & 63, e >> 12 & 63);
         const T* m0 = mat + 9 * (int)idh[q];
-        v.R[0] = mul(p.iAx[cc.j + (long long)cc.k * Ny], m0[3]);
-        v.R[1] = mul(p.iAy[cc.i + (long long)cc.k * Nx], m0[4]);
-        v.R[2] = mul(p.iAz[cc.i + (long long)cc.j * Nx], m0[5]);
+        v.R[0] = mul(__ldg(p.iAx + cc.j + (long long)cc.k * Ny), m0[3]);
+        v.R[1] = mul(__ldg(p.iAy + cc.i + (long long)cc.k * Nx), m0[4]);
+        v.R[2] = mul(__ldg(p.iAz + cc.i + (long long)cc.j * Nx), m0[5]);
         ColumnInv<T, 1> ci;
         ci.init(p, cc.i, cc.j);
         f = ci.at(p, cc.k);
@@ -552,20 +440,8 @@ k_loop(FitParams<T> p, LoopTiling tl, int n_steps, long long step0, unsigned* sy
     Eo = sw;
     __syncthreads();
   }
-  // the last block to leave sets the words back for the next launch
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    if (atomicAdd(sync + kSyncDone, 1u) == gridDim.x - 1) {
-      __threadfence();
-      atomicExch(sync + kSyncCount, 0u);
-      atomicExch(sync + kSyncAbort, 0u);
-      atomicExch(sync + kSyncDone, 0u);
-    }
-  }
+  loop_leave(sync);
 }
-
-namespace {
 
 int loop_sms() {
   static int sms[64];
@@ -579,11 +455,10 @@ int loop_sms() {
   return sms[dev];
 }
 
-// The split whose largest tile takes the fewest cell updates per step: H on
-// the tile and its low halo, E on the tile, the halo's loads (x faces count
-// twice: a sector per cell).  nbx = 0 when no split fits.  The search takes
-// tens of microseconds, as long as several steps, so each thread keeps the
-// answer of its last shape.
+namespace {
+
+// The tile split of a grid.  The search takes tens of microseconds, as long as
+// several steps, so each thread keeps the answer of its last shape.
 template <typename T>
 LoopTiling loop_tiling(const FitParams<T>& p, int sms) {
   struct Last { int Nx, Ny, Nz, n_mat, sms; LoopTiling tl; };
@@ -591,22 +466,10 @@ LoopTiling loop_tiling(const FitParams<T>& p, int sms) {
   const int mats = p.n_mat <= kLoopMat ? p.n_mat : (p.n_mat <= 256 ? 256 : 65536);
   if (last.Nx == p.Nx && last.Ny == p.Ny && last.Nz == p.Nz && last.n_mat == mats && last.sms == sms)
     return last.tl;
-  LoopTiling best = {0, 0, 0, 0, 0, 0};
-  double best_cost = 0;
   const int idb = p.n_mat <= 256 ? 1 : 2;
-  for (int nx = 1; nx <= sms && nx <= p.Nx; nx++)
-    for (int ny = 1; nx * ny <= sms && ny <= p.Ny; ny++) {
-      const int nz = sms / (nx * ny) < p.Nz ? sms / (nx * ny) : p.Nz;
-      const int tx = (p.Nx + nx - 1) / nx, ty = (p.Ny + ny - 1) / ny, tz = (p.Nz + nz - 1) / nz;
-      if (tx > kLoopDim || ty > kLoopDim || tz > kLoopDim) continue;
-      const LoopLayout<T> lay(tx, ty, tz, p.n_mat, idb);
-      if (lay.bytes > kLoopSmem) continue;
-      const double cost = lay.n_ext + lay.n_own + 0.5 * lay.n_shell + 1.0 * ty * tz;
-      if (best.nbx == 0 || cost < best_cost) {
-        best = {nx, ny, nz, tx, ty, tz};
-        best_cost = cost;
-      }
-    }
+  const LoopTiling best = loop_search(p.Nx, p.Ny, p.Nz, sms, [&](int tx, int ty, int tz) {
+    return LoopLayout<T>(tx, ty, tz, p.n_mat, idb);
+  });
   last = {p.Nx, p.Ny, p.Nz, mats, sms, best};
   return best;
 }

@@ -42,9 +42,9 @@ struct ColumnInv {
     const int jx = wx ? jn : j;
     dkx = (wx && wy) ? 1 : 0;
     dky = wy ? 1 : 0;
-    Lx = lx[i];
-    Ly = ly[j];
-    LyX = ly[jx];
+    Lx = __ldg(lx + i);
+    Ly = __ldg(ly + j);
+    LyX = __ldg(ly + jx);
     if (!has) {
       bits = 127;
       return;

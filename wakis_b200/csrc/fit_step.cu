@@ -9,10 +9,33 @@
 
 #include "../../include/wakis_b200.h"
 #include "abi_internal.h"
+#include "fit_comp.cuh"
 #include "fit_common.cuh"
 #include "fit_kernels.cuh"
 
 using namespace wk;
+
+thread_local KernelTimer* g_kernel_timer = nullptr;
+
+// Small grids: all steps in one launch where the tiles fit the shared memory
+// of the SMs (about 430k FP64, 860k FP32, 450k to 600k FP32c cells).  A call pays
+// for filling them once (us: 13 + 9e-5 N) and then less a step.  Break-even
+// against the per-step kernels, measured on B200 in steps a call: where a step
+// is several launches (open ends, PMC or periodic faces; FP32c rows that no
+// TMA box takes) 0.7 to 3.7 over the whole range (FP64 16x16x24 open 0.7,
+// 55x61x110 open 2.3, FP32 176x24x143 open 3.7, FP32c 55x61x110 1.7): from 4
+// steps on.  Where every face is PEC-masked a step is one launch of 10 to 18
+// us, and the break-even goes with N: 16x16x24 1.8, 40x40x80 FP64 / FP32 /
+// FP32c 3.9 / 3.2 / 3.7, 60x60x60 8.4 / 5.0 / 6.2, 64x64x96 FP32 8.6, FP32c
+// 14.3, 176x24x143 FP32 13.6: from N / 25000 steps on.
+bool wk_one_launch_call(const wk_fit_desc* d, int n_steps) {
+  if (d->kernel != WK_KERNEL_AUTO || !d->sync || n_steps < 4 || d->steps_per_launch != 0 ||
+      g_kernel_timer)
+    return false;
+  bool closed = d->has_pec && !d->has_pmc && (d->dtype != WK_F32C || d->Nx % 4 == 0);
+  for (int f = 0; f < 6; f++) closed = closed && d->pec_face[f] == 0;
+  return !closed || (long long)d->Nx * d->Ny * d->Nz <= 25000LL * n_steps;
+}
 
 namespace {
 
@@ -95,14 +118,7 @@ int run_fused(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_t s
   int par = d->par;
   const bool big = d->Nx >= 5 && d->Ny >= 5 && d->Nz >= 5 && d->Nz - 4 <= 65535 &&
                    (d->Ny - 4 + 1) / 2 <= 65535;
-  // small grids: all steps in one launch where the tiles fit the shared
-  // memory of the SMs (about 430k FP64 or 860k FP32 cells).  From 4 steps on
-  // it is the faster one over the whole range, set-up included: 4 steps of
-  // 16x16x24 FP64 25 against 42 us, 40x40x80 FP64 51 / 100, 55x61x110 FP64
-  // 102 / 189, 64x64x160 FP32 132 / 126; 8 steps 37 / 83, 79 / 199, 158 / 377,
-  // 192 / 251; 2 steps of 64x64x160 100 / 67.
-  if (d->kernel == WK_KERNEL_AUTO && big && d->sync && n_steps >= 4 && d->steps_per_launch == 0 &&
-      !g_kernel_timer) {
+  if (wk_one_launch_call(d, n_steps) && big) {
     const FitParams<T> p = make_params<T>(d, par);
     if (loop_supported<T>(p)) {
       cudaError_t e = launch_loop<T>(p, n_steps, step0, d->sync, st);
@@ -186,6 +202,18 @@ int run_split(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_t s
 
 }  // namespace
 
+extern "C" int wk_fit_one_launch(const wk_fit_desc* d, int n_steps) {
+  if (wk_validate_fit(d, "wk_fit_one_launch") || !wk_one_launch_call(d, n_steps) || d->Nx < 5 ||
+      d->Ny < 5 || d->Nz < 5)
+    return 0;
+  if (d->dtype == WK_F32C) {
+    const FitParams<double> p = make_params<double>(d, d->par);
+    return !d->comp_stencil && d->j_mode != WK_J_ARRAY && loop_comp_supported(p);
+  }
+  return d->dtype == WK_F64 ? loop_supported<double>(make_params<double>(d, d->par))
+                            : loop_supported<float>(make_params<float>(d, d->par));
+}
+
 extern "C" int wk_zero_ghosts(const wk_fit_desc* d, void* stream) {
   int rc = wk_validate_fit(d, "wk_zero_ghosts");
   if (rc) return rc;
@@ -238,8 +266,6 @@ extern "C" int wk_fit_step(const wk_fit_desc* d, int n_steps, long long step0, v
   return d->dtype == WK_F64 ? run_fused<double>(d, n_steps, step0, st)
                             : run_fused<float>(d, n_steps, step0, st);
 }
-
-thread_local KernelTimer* g_kernel_timer = nullptr;
 
 namespace {
 __global__ void k_counter_add(long long* ctr, long long inc) { *ctr += inc; }
