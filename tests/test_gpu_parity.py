@@ -255,6 +255,43 @@ def test_tma_on_row_groups_equals_twopass(dtype, precision_shape, rows, bcs):
     assert torch.equal(ha, hb)
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shape", [(8, 5, 5), (12, 7, 6), (36, 33, 9)])
+@pytest.mark.parametrize("bcs", [(["pec", "pec", "abc"], ["pec", "pec", "abc"]),
+                                 (["periodic", "periodic", "pec"], ["periodic", "periodic", "pml"]),
+                                 (["pmc", "pec", "abc"], ["pec", "pmc", "pec"])])
+def test_tma_shell_beside_tiles_equals_cell_kernel(dtype, shape, bcs):
+    """The shell of a TMA step, formed beside the tiles from the old state
+    alone: fields, stored J and Ez history of the per-cell kernel value for
+    value, from random fields on every entry, also with J stored as an array,
+    down to grids that are all shell but one cell."""
+    import wakis_b200 as wb
+    from wakis_b200.sources import Beam
+    sol = []
+    for kernel in ("tma", "cell"):
+        g = wb.GridFIT3D(-0.03, 0.031, -0.02, 0.022, -0.04, 0.043, *shape, verbose=0)
+        m = np.zeros(shape, bool)
+        m[1:5, :, 2:4] = True
+        g.add_solid("a", m, [4.0, 1.0, 10.0])
+        s = wb.SolverFIT3D(g, bc_low=bcs[0], bc_high=bcs[1], dtype=dtype, bg=[1.0, 1.0, 0.5],
+                           use_stl=True, use_sibc=False, verbose=0, n_pml=1)
+        s.kernel = kernel
+        rng = np.random.default_rng(11)
+        s._first_step()
+        s.E.fromarray(300 * rng.standard_normal(3 * s.N))
+        s.H.fromarray(rng.standard_normal(3 * s.N))
+        h = torch.zeros((9, s.Nz, 6), dtype=s._cap_dtype, device="cuda")
+        bp = Beam(q=1e-9, sigmaz=0.005).params(s)
+        s._advance(3, 0, beam=bp, capture=(h, 1, 1, 3, 3))
+        s._materialize_J()
+        s._advance(3, 3, beam=bp, capture=(h, 1, 1, 3, 3))
+        s.check_status()
+        sol.append((s, h))
+    (a, ha), (b, hb) = sol
+    assert torch.equal(a.E.array, b.E.array) and torch.equal(a.H.array, b.H.array)
+    assert torch.equal(a._J, b._J) and torch.equal(ha, hb)
+
+
 @pytest.mark.parametrize("shape", [(7, 5, 9), (16, 13, 40), (67, 9, 23), (33, 41, 57)])
 @pytest.mark.parametrize("idx", VALID)
 def test_many_steps_per_launch_equal_cell_kernel(idx, shape):

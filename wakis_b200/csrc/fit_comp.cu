@@ -209,6 +209,7 @@ k_e_comp_cs(FitParams<double> p, CompState st, long long step) {
 // cell per thread (comp_shell_h / comp_shell_e, fit_comp.cuh).
 __global__ void __launch_bounds__(kShellBlock) k_h_comp_shell(FitParams<double> p, CompState st,
                                                                ShellGrid g) {
+  pdl_trigger();
   Cell c;
   if (!shell_cell_of(g, blockIdx.x, threadIdx.x, p.Nx, p.Ny, p.Nz, c)) return;
   comp_shell_h(p, st, c);
@@ -289,17 +290,16 @@ int wk_comp_step(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_
     FitParams<double> p = make_params<double>(d, par);
     CompState cs = comp_state(d, par);
     if (tma) {
-      // fused step (whole grid when every face is PEC-masked, else the
-      // interior, then the shell: H from the old state, E from the new H)
+      // fused step: the whole grid when every face is PEC-masked, else the
+      // interior beside the H of the shell (both from the old state), then the
+      // E of the shell from the new H
+      const int mode = tma_comp_mode(p);
+      const ShellGrid g2 = shell_grid(d->Nx, d->Ny, d->Nz, mode == 2);
+      const unsigned sb2 = (unsigned)(g2.nbA + g2.nbB + g2.nbC);
+      if (mode != 1) k_h_comp_shell<<<sb2, kShellBlock, 0, st>>>(p, cs, g2);
       cudaError_t e = launch_tma_comp(d, p, par, step0 + s, st, d->tile_planes);
       if (e != cudaSuccess) return wk_fail(-(int)e, "wk_fit_step: %s", cudaGetErrorString(e));
-      const int mode = tma_comp_mode(p);
-      if (mode != 1) {
-        const ShellGrid g2 = shell_grid(d->Nx, d->Ny, d->Nz, mode == 2);
-        const unsigned sb2 = (unsigned)(g2.nbA + g2.nbB + g2.nbC);
-        k_h_comp_shell<<<sb2, kShellBlock, 0, st>>>(p, cs, g2);
-        k_e_comp_shell<<<sb2, kShellBlock, 0, st>>>(p, cs, step0 + s, g2);
-      }
+      if (mode != 1) k_e_comp_shell<<<sb2, kShellBlock, 0, st>>>(p, cs, step0 + s, g2);
     } else {
       timer_begin(st);
       if (cstencil) k_h_comp_cs<<<grid, blk, 0, st>>>(p, cs);

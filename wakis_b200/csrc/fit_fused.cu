@@ -5,12 +5,12 @@
 // no face mask reaches any row they need) with single-coefficient rows, and
 // the two-cell shell with the general row code (masks, wraps, grid edges).
 // It serves grids the TMA kernel cannot take and is the cross-check of the
-// TMA schedule.  The shell kernels here also close the TMA step when a face
-// is not PEC-masked.
+// TMA schedule, whose shell k_shell_step steps when a face is not PEC-masked.
 #include "../../include/wakis_b200.h"
 #include "abi_internal.h"
 #include "fit_common.cuh"
 #include "fit_kernels.cuh"
+#include "fit_rows.cuh"
 
 namespace wk {
 
@@ -161,8 +161,8 @@ k_e_pass(FitParams<T> p, long long step, int mat_smem) {
   }
 }
 
-// Shell launches of the two-pass and TMA schedules (decomposition in
-// fit_kernels.cuh: ShellGrid).
+// Shell launches of the two-pass schedule (decomposition in fit_kernels.cuh:
+// ShellGrid).
 template <typename T>
 __global__ void __launch_bounds__(kShellThreads) k_h_shell(FitParams<T> p, ShellGrid g) {
   Cell c;
@@ -258,19 +258,162 @@ cudaError_t launch_two_pass(const FitParams<T>& p, long long step, cudaStream_t 
   return cudaGetLastError();
 }
 
+// Shell of a TMA step: the new H of the cell and of its three backward
+// neighbours from the old state (9 rows; branch-free, the column factors carry
+// the masks), then the new E of the cell.  Nothing is read that another kernel
+// of the step writes, so the tile kernel runs beside it.  Bound by its
+// instructions (1700 a warp) on z planes, on x faces by the sectors of which it
+// uses two cells.  Measured on B200, H launch, E launch and tiles in turn / this
+// beside the tiles (us a step): open ends 96x96x240 FP64 64.2 / 53.7, FP32 54.1 /
+// 43.7, 64x64x400 FP64 52.1 / 41.6, 149x131x301 FP64 160.6 / 150.1, 256x200x500
+// 470 / 463; periodic 96x96x240 FP64 with J stored 152 / 113.  Slower forms of
+// it, same order: planes of a column one after another in a thread 58.2 (96x96x240
+// FP64), a component of E per thread 52.2 there but 154.3 for 149x131x301.
+constexpr int kShellStep = 128;
+
 template <typename T>
-cudaError_t launch_shell_pair(const FitParams<T>& p, long long step, cudaStream_t st,
+__global__ void __launch_bounds__(kShellStep, 4)
+k_shell_step(FitParams<T> p, long long step, int total) {
+  pdl_trigger();
+  const int idx = blockIdx.x * kShellStep + threadIdx.x;
+  if (idx >= total) return;
+  step = step_index(p, step);
+  const int Nx = p.Nx, Ny = p.Ny, Nz = p.Nz, N = (int)p.N, NxNy = (int)p.NxNy;
+  const Cell c = shell_cell(idx, Nx, Ny, Nz);
+  const int n = c.i + c.j * Nx + c.k * NxNy;
+  const bool vx = n >= 1, vy = n >= Nx, vz = n >= NxNy;
+  // backward neighbours; one outside the grid has H = 0, its row is formed at
+  // the cell itself
+  const Cell cx = vx ? minus_x(c, Nx, Ny) : c, cy = vy ? minus_y(c, Ny) : c;
+  const int kz = vz ? c.k - 1 : c.k;
+  const int mx = vx ? n - 1 : n, my = vy ? n - Nx : n, mz = vz ? n - NxNy : n;
+  const T* const ex = p.E_in;
+  const T* const ey = ex + p.N;
+  const T* const ez = ey + p.N;
+  const T* const hx = p.H_in;
+  const T* const hy = hx + p.N;
+  const T* const hz = hy + p.N;
+  auto ld = [&](const T* f, int q) { return q < N ? __ldg(f + q) : T(0); };
+  const int id = load_id(p.mat_id, p.id_bytes, n);
+  const int idx_ = load_id(p.mat_id, p.id_bytes, mx), idy = load_id(p.mat_id, p.id_bytes, my),
+            idz = load_id(p.mat_id, p.id_bytes, mz);
+  const T ex0 = __ldg(ex + n), ey0 = __ldg(ey + n), ez0 = __ldg(ez + n);
+  const T ey1 = ld(ey, n + 1), ez1 = ld(ez, n + 1);
+  const T ex2 = ld(ex, n + Nx), ez2 = ld(ez, n + Nx);
+  const T ex3 = ld(ex, n + NxNy), ey3 = ld(ey, n + NxNy);
+  T h0 = __ldg(hx + n), h1 = __ldg(hy + n), h2 = __ldg(hz + n);
+  // x neighbour: rows y, z; y neighbour: rows x, z; z neighbour: rows x, y
+  const T xex = __ldg(ex + mx), xey = __ldg(ey + mx), xez = __ldg(ez + mx);
+  const T xex2 = ld(ex, mx + Nx), xex3 = ld(ex, mx + NxNy);
+  T xhx = T(0), xhy = __ldg(hy + mx), xhz = __ldg(hz + mx);
+  const T yex = __ldg(ex + my), yey = __ldg(ey + my), yez = __ldg(ez + my);
+  const T yey1 = ld(ey, my + 1), yey3 = ld(ey, my + NxNy);
+  T yhx = __ldg(hx + my), yhy = T(0), yhz = __ldg(hz + my);
+  const T zex = __ldg(ex + mz), zey = __ldg(ey + mz), zez = __ldg(ez + mz);
+  const T zez1 = ld(ez, mz + 1), zez2 = ld(ez, mz + Nx);
+  T zhx = __ldg(hx + mz), zhy = __ldg(hy + mz), zhz = T(0);
+  const bool desc = p.h_desc != 0;
+  const T z = T(0);
+  auto imu = [&](int m, int d) { return __ldg(p.mat + 9 * m + 3 + d); };
+  auto pmc = [&](T R, int d, int i, int j, int k) {
+    return p.has_pmc && !face_val(p.pmc_face, d, i, j, k, Nx, Ny, Nz) ? T(0) : R;
+  };
+  // two cells and more from the x and y faces only the z faces matter: the
+  // columns of all rows differ in the lengths alone (z planes of 149x131: 14.4 us,
+  // without this form 17.1)
+  const bool inner = c.i >= 2 && c.i <= Nx - 3 && c.j >= 2 && c.j <= Ny - 3;
+  ColumnInv<T, 1> ci;
+  RowCols<T> co, cz;
+  if (inner) {
+    ci.Lx = __ldg(p.Lx + c.i);
+    ci.Ly = ci.LyX = __ldg(p.Ly + c.j);
+    ci.bits = 127;
+    ci.dkx = ci.dky = 0;
+  } else {
+    ci.init(p, c.i, c.j);
+  }
+  co = ci.at(p, c.k);
+  h_rows(p.dt, desc, pmc(mul(__ldg(p.iAx + c.j + c.k * Ny), imu(id, 0)), 0, c.i, c.j, c.k),
+         pmc(mul(__ldg(p.iAy + c.i + c.k * Nx), imu(id, 1)), 1, c.i, c.j, c.k),
+         pmc(mul(__ldg(p.iAz + c.i + c.j * Nx), imu(id, 2)), 2, c.i, c.j, c.k), co, ex0, ey0, ez0,
+         ey1, ez1, ex2, ez2, ex3, ey3, h0, h1, h2);
+  cz = ci.at(p, kz);
+  h_rows(p.dt, desc, pmc(mul(__ldg(p.iAx + c.j + kz * Ny), imu(idz, 0)), 0, c.i, c.j, kz),
+         pmc(mul(__ldg(p.iAy + c.i + kz * Nx), imu(idz, 1)), 1, c.i, c.j, kz), z, cz, zex, zey, zez,
+         z, zez1, z, zez2, ex0, ey0, zhx, zhy, zhz);
+  const bool ko = co.xO != z, kup = co.xZ != z;   // z-face masks of the inner cells
+  if (inner) {
+    cz = co;
+    const T l = __ldg(p.Lx + c.i - 1);
+    cz.xO = cz.xY = ko ? l : z;
+    cz.xZ = kup ? l : z;
+  } else {
+    ci.init(p, cx.i, cx.j);
+    cz = ci.at(p, cx.k);
+  }
+  h_rows(p.dt, desc, z, pmc(mul(__ldg(p.iAy + cx.i + cx.k * Nx), imu(idx_, 1)), 1, cx.i, cx.j, cx.k),
+         pmc(mul(__ldg(p.iAz + cx.i + cx.j * Nx), imu(idx_, 2)), 2, cx.i, cx.j, cx.k), cz, xex, xey,
+         xez, ey0, ez0, xex2, z, xex3, z, xhx, xhy, xhz);
+  if (inner) {
+    cz = co;
+    const T l = __ldg(p.Ly + c.j - 1);
+    cz.yO = cz.yX = ko ? l : z;
+    cz.yZ = kup ? l : z;
+  } else {
+    ci.init(p, cy.i, cy.j);
+    cz = ci.at(p, cy.k);
+  }
+  h_rows(p.dt, desc, pmc(mul(__ldg(p.iAx + cy.j + cy.k * Ny), imu(idy, 0)), 0, cy.i, cy.j, cy.k), z,
+         pmc(mul(__ldg(p.iAz + cy.i + cy.j * Nx), imu(idy, 2)), 2, cy.i, cy.j, cy.k), cz, yex, yey,
+         yez, yey1, z, ex0, ez0, z, yey3, yhx, yhy, yhz);
+  const T* const m0 = p.mat + 9 * id;
+  const T ie[3] = {__ldg(m0), __ldg(m0 + 1), __ldg(m0 + 2)};
+  auto efac = [&](T itA, int d) -> T {
+    const T R = mul(ie[d], itA);
+    return p.has_pec && !face_val(p.pec_face, d, c.i, c.j, c.k, Nx, Ny, Nz) ? T(0) : R;
+  };
+  ColumnInv<T, -1> cj;
+  if (inner) {
+    cj.Lx = __ldg(p.tLx + c.i);
+    cj.Ly = cj.LyX = __ldg(p.tLy + c.j);
+    cj.bits = 127;
+    cj.dkx = cj.dky = 0;
+  } else {
+    cj.init(p, c.i, c.j);
+  }
+  T curl[3];
+  e_rows(efac(__ldg(p.itAx + c.j + c.k * Ny), 0), efac(__ldg(p.itAy + c.i + c.k * Nx), 1),
+         efac(__ldg(p.itAz + c.i + c.j * Nx), 2), cj.at(p, c.k), h0, h1, h2, vx ? xhy : z,
+         vx ? xhz : z, vy ? yhx : z, vy ? yhz : z, vz ? zhx : z, vz ? zhy : z, curl[0], curl[1],
+         curl[2]);
+  const T eold[3] = {ex0, ey0, ez0};
+  if (p.cap_on) capture(p, c, n, step, ez0);
+  T jv[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) jv[d] = j_in(p, d, c, n, step, eold[d], __ldg(m0 + 6 + d));
+  p.H_out[n] = h0;
+  p.H_out[p.N + n] = h1;
+  p.H_out[2 * p.N + n] = h2;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const T enew = add(eold[d], mul(p.dt, sub(curl[d], mul(ie[d], jv[d]))));
+    p.E_out[d * p.N + n] = enew;
+    if (p.j_mode == WK_J_ARRAY && p.use_cond) p.J[d * p.N + n] = mul(__ldg(m0 + 6 + d), enew);
+  }
+}
+
+template <typename T>
+cudaError_t launch_shell_step(const FitParams<T>& p, long long step, cudaStream_t st,
                               bool planes_only) {
-  const ShellGrid sg = shell_grid(p.Nx, p.Ny, p.Nz, planes_only);
-  const unsigned sb = (unsigned)(sg.nbA + sg.nbB + sg.nbC);
-  k_h_shell<T><<<sb, kShellThreads, 0, st>>>(p, sg);
-  k_e_shell<T><<<sb, kShellThreads, 0, st>>>(p, step, sg);
+  const int total = (int)shell_cells(p.Nx, p.Ny, p.Nz, planes_only);
+  k_shell_step<T><<<(unsigned)((total + kShellStep - 1) / kShellStep), kShellStep, 0, st>>>(p, step,
+                                                                                           total);
   return cudaGetLastError();
 }
 
-template cudaError_t launch_shell_pair<double>(const FitParams<double>&, long long, cudaStream_t,
+template cudaError_t launch_shell_step<double>(const FitParams<double>&, long long, cudaStream_t,
                                                bool);
-template cudaError_t launch_shell_pair<float>(const FitParams<float>&, long long, cudaStream_t,
+template cudaError_t launch_shell_step<float>(const FitParams<float>&, long long, cudaStream_t,
                                               bool);
 
 template cudaError_t launch_two_pass<double>(const FitParams<double>&, long long, cudaStream_t,

@@ -127,38 +127,62 @@ inline FitParams<T> make_params(const wk_fit_desc* d, int par) {
 }
 
 
-// Cell of the idx-th shell cell: planes k in {0,1,Nz-2,Nz-1}, then rows
-// j in {0,1,Ny-2,Ny-1} of the inner planes, then columns i in
-// {0,1,Nx-2,Nx-1} of the inner rows (needs Nx, Ny, Nz >= 5).
-__device__ __forceinline__ Cell shell_cell(long long idx, int Nx, int Ny, int Nz) {
+// Cell of the idx-th shell cell (idx < shell_cells): planes k in {0, 1, Nz-2,
+// Nz-1}, then rows j in {0, 1, Ny-2, Ny-1} of the inner planes, then columns i in
+// {0, 1, Nx-2, Nx-1} of the inner rows (needs Nx, Ny, Nz >= 5, cells < 2^31).
+inline long long shell_cells(int Nx, int Ny, int Nz, bool planes_only) {
+  const long long planes = 4LL * Nx * Ny;
+  return planes_only ? planes : planes + 4LL * (Nz - 4) * (Nx + Ny - 4);
+}
+__device__ __forceinline__ Cell shell_cell(int idx, int Nx, int Ny, int Nz) {
   Cell c;
-  const long long NxNy = (long long)Nx * Ny;
-  const long long A = 4 * NxNy;
-  if (idx < A) {
-    const int kk = (int)(idx / NxNy);
-    const long long rem = idx - kk * NxNy;
+  const int NxNy = Nx * Ny;
+  if (idx < 4 * NxNy) {
+    const int kk = idx / NxNy, rem = idx - kk * NxNy;
     c.k = kk < 2 ? kk : Nz - 4 + kk;
-    c.j = (int)(rem / Nx);
-    c.i = (int)(rem - (long long)c.j * Nx);
+    c.j = rem / Nx;
+    c.i = rem - c.j * Nx;
     return c;
   }
-  idx -= A;
-  const long long B = 4LL * Nx * (Nz - 4);
-  if (idx < B) {
-    const long long t = idx / Nx;
-    c.i = (int)(idx - t * Nx);
-    const int jj = (int)(t % 4);
-    c.j = jj < 2 ? jj : Ny - 4 + jj;
-    c.k = 2 + (int)(t / 4);
+  idx -= 4 * NxNy;
+  if (idx < 4 * Nx * (Nz - 4)) {
+    const int t = idx / Nx;
+    c.i = idx - t * Nx;
+    c.j = (t & 3) < 2 ? (t & 3) : Ny - 4 + (t & 3);
+    c.k = 2 + (t >> 2);
     return c;
   }
-  idx -= B;
-  const int ii = (int)(idx % 4);
-  c.i = ii < 2 ? ii : Nx - 4 + ii;
-  const long long t = idx / 4;
-  c.j = 2 + (int)(t % (Ny - 4));
-  c.k = 2 + (int)(t / (Ny - 4));
+  idx -= 4 * Nx * (Nz - 4);
+  c.i = (idx & 3) < 2 ? (idx & 3) : Nx - 4 + (idx & 3);
+  const int t = idx >> 2, kk = t / (Ny - 4);
+  c.k = 2 + kk;
+  c.j = 2 + t - kk * (Ny - 4);
   return c;
+}
+
+// A launch that may start once every block of the kernel before it in the
+// stream has passed pdl_trigger (or ended); pdl_wait ends when that kernel has
+// ended and its writes are visible.  A kernel before it that was launched the
+// ordinary way has seen everything earlier in the stream complete, so the
+// blocks of both may read what those wrote.
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t launch_beside(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st,
+                          A... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // Fused step of one cell with the general row code: the new H of the cell
@@ -222,12 +246,12 @@ __device__ __forceinline__ void fused_cell_general(const FitParams<T>& p, long l
 template <typename T>
 cudaError_t launch_two_pass(const FitParams<T>& p, long long step, cudaStream_t st, int kb);
 
-// Shell of a step whose interior was stepped by a fused kernel: H of the
-// shell cells from the old state, then E of the shell cells from the new H
-// (fit_fused.cu); needs Nx, Ny, Nz >= 5 and the interior H_out written.
+// Step of the shell cells (planes_only: of the four z-boundary planes) from the
+// old state, in one launch that lets a launch_beside one start with it
+// (fit_fused.cu); needs Nx, Ny, Nz >= 5, cells < 2^31, separate old and new state.
 template <typename T>
-cudaError_t launch_shell_pair(const FitParams<T>& p, long long step, cudaStream_t st,
-                              bool planes_only = false);
+cudaError_t launch_shell_step(const FitParams<T>& p, long long step, cudaStream_t st,
+                              bool planes_only);
 
 // TMA-staged fused step (fit_tma.cu): interior tiles + shell launches.
 template <typename T>
@@ -235,9 +259,6 @@ bool tma_supported(const FitParams<T>& p);
 // Row and component pitch of 16 bytes.
 template <typename T>
 bool tma_pitch(const FitParams<T>& p);
-// Faster than the two-pass schedule on this grid.
-template <typename T>
-bool tma_preferred(const FitParams<T>& p);
 template <typename T>
 cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
                        int rows);

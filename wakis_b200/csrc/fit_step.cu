@@ -20,21 +20,23 @@ thread_local KernelTimer* g_kernel_timer = nullptr;
 // Small grids: all steps in one launch where the tiles fit the shared memory
 // of the SMs (about 430k FP64, 860k FP32, 450k to 600k FP32c cells).  A call pays
 // for filling them once (us: 13 + 9e-5 N) and then less a step.  Break-even
-// against the per-step kernels, measured on B200 in steps a call: where a step
-// is several launches (open ends, PMC or periodic faces; FP32c rows that no
-// TMA box takes) 0.7 to 3.7 over the whole range (FP64 16x16x24 open 0.7,
-// 55x61x110 open 2.3, FP32 176x24x143 open 3.7, FP32c 55x61x110 1.7): from 4
-// steps on.  Where every face is PEC-masked a step is one launch of 10 to 18
-// us, and the break-even goes with N: 16x16x24 1.8, 40x40x80 FP64 / FP32 /
-// FP32c 3.9 / 3.2 / 3.7, 60x60x60 8.4 / 5.0 / 6.2, 64x64x96 FP32 8.6, FP32c
-// 14.3, 176x24x143 FP32 13.6: from N / 25000 steps on.
+// against the per-step kernels, measured on B200 in steps a call: FP32c with
+// open ends or rows that no TMA box takes (three and four launches a step) 0.7
+// to 3.5 over the whole range (55x61x110 1.6, 64x64x96 3.3): from 4 steps on.
+// Other grids with a face that is not PEC-masked, two launches a step of 10 to 30
+// us: FP64 16x16x24 1.2, 40x40x80 3.8, 55x61x110 4.4, FP32 48x48x100 4.5,
+// 64x64x160 9.1: from N / 50000 steps on.  Every face PEC-masked, one launch of
+// 10 to 18 us: 16x16x24 1.8, 40x40x80 FP64 / FP32 / FP32c 3.9 / 3.2 / 3.7,
+// 60x60x60 8.4 / 5.0 / 6.2, 64x64x96 FP32 8.6, FP32c 14.3, 176x24x143 FP32
+// 13.6: from N / 25000 steps on.
 bool wk_one_launch_call(const wk_fit_desc* d, int n_steps) {
   if (d->kernel != WK_KERNEL_AUTO || !d->sync || n_steps < 4 || d->steps_per_launch != 0 ||
       g_kernel_timer)
     return false;
-  bool closed = d->has_pec && !d->has_pmc && (d->dtype != WK_F32C || d->Nx % 4 == 0);
+  bool closed = d->has_pec && !d->has_pmc;
   for (int f = 0; f < 6; f++) closed = closed && d->pec_face[f] == 0;
-  return !closed || (long long)d->Nx * d->Ny * d->Nz <= 25000LL * n_steps;
+  if (d->dtype == WK_F32C && (!closed || d->Nx % 4 != 0)) return true;
+  return (long long)d->Nx * d->Ny * d->Nz <= (closed ? 25000LL : 50000LL) * n_steps;
 }
 
 namespace {
@@ -133,7 +135,7 @@ int run_fused(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_t s
     const bool ok = tma_supported<T>(p0) && tma_supported<T>(p1);
     if (d->kernel == WK_KERNEL_TMA && !(ok && tma_pitch<T>(p0)))
       return wk_fail(WK_E_SHAPE, "wk_fit_step: TMA kernel needs a 16-byte row pitch, dims >= 5");
-    use_tma = ok && (d->kernel == WK_KERNEL_TMA || tma_preferred<T>(p0));
+    use_tma = ok;
   }
   if (use_tma) {
     int s = 0;

@@ -1,7 +1,7 @@
 // Fused FIT step with TMA-staged plane tiles (sm_100a).
 //
 // Which cells a launch covers depends on the face mode (MODE, see k_tma): the
-// interior (2 <= i, j, k <= N-3, the two-cell shell in separate launches),
+// interior (2 <= i, j, k <= N-3, the two-cell shell in a launch beside),
 // all of x and y for 2 <= k <= Nz-3 (x/y faces PEC-masked), or the whole grid
 // (every face PEC-masked).  Block (bx, by, bz) owns the tile
 // i in [i0, i0+TX), j in [j0, j0+TY) of planes [k0, k0+KC) and marches in z;
@@ -168,7 +168,7 @@ __device__ __forceinline__ RowEntry<T> row_entry(const FitParams<T>& p, int r, i
 // ids are one byte each; the table reads are then shared-memory loads.  JM: the J mode of the launch
 // (WK_J_ZERO, WK_J_SIGMA_E or WK_J_ARRAY), fixed at compile time.
 // MODE 0: interior cells only (2 <= i, j, k <= N-3), the two-cell shell runs
-// in separate launches.  MODE 1: every face of the grid carries the PEC
+// in a launch beside this one.  MODE 1: every face of the grid carries the PEC
 // column mask (pec, electric or pml on all six faces, no PMC); the tiles
 // cover the whole grid and the cells next to a face use the same
 // single-coefficient rows with the masked terms set to zero: an E entry
@@ -176,10 +176,10 @@ __device__ __forceinline__ RowEntry<T> row_entry(const FitParams<T>& p, int r, i
 // to its face gets no curl.  The neighbours that the flat-offset operators
 // reach by wrapping (i+1 past Nx-1, j+1 past Ny-1) are tangential to the
 // opposite face, so every wrapped term is masked and no shell launch
-// follows.  MODE 2: the four x/y faces are PEC-masked and the z faces are
+// is needed.  MODE 2: the four x/y faces are PEC-masked and the z faces are
 // not (ABC, periodic): the tiles cover all of x and y for the planes
-// 2 <= k <= Nz-3 (no z face is involved there), and the shell launches
-// cover only the planes k in {0, 1, Nz-2, Nz-1}.  Warps with no cell on or
+// 2 <= k <= Nz-3 (no z face is involved there), and the shell launch
+// covers only the planes k in {0, 1, Nz-2, Nz-1}.  Warps with no cell on or
 // next to a face take the unmasked rows.
 // GRP: row groups (see TmaMaps); lg = log2 of the rows per group.
 template <typename T, bool SM, int JM, int MODE, bool DESC, bool GRP, int TW>
@@ -457,6 +457,16 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
       if (issue_wh && pl + kHS - 1 <= k1 - 1) issue_h(pl + kHS - 1);
     };
     if (!LATE && (issue_we || issue_wh) && !prologue) issue_next();
+    // the stored J of the owned cells, read ahead of the stores of the E phase
+    // (read at each row's use 100 us a launch, 96x96x240 periodic; so 70)
+    T jr[2][3];
+    if (JM == WK_J_ARRAY && !prologue) {
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+          if (eval[r]) jr[r][d] = p.J[d * N + cn0 + (pl - pstart) * NxNy + dcell * r];
+    }
     // prefetch the ids of plane pl+1
     const bool more = pl + 1 < k1;
     int idn[2] = {0, 0};
@@ -611,7 +621,7 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
           // J entering the row (the j_in rules with the mode fixed)
           T jv = T(0);
           if (JM == WK_J_SIGMA_E) jv = mul(sigma, eold[d]);
-          if (JM == WK_J_ARRAY) jv = p.J[d * N + n];
+          if (JM == WK_J_ARRAY) jv = jr[r][d];
           if (d == 2 && (cell_bits & (4 << r))) jv = j_in(p, d, cc, n, step, eold[d], sigma);
           const T enew = add(eold[d], mul(p.dt, sub(curl[d], mul(ieps, jv))));
           (d == 0 ? eq : (d == 1 ? eq1 : eq1 + N))[dcell * r] = enew;
@@ -642,6 +652,7 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
     }
     __syncthreads();
   }
+  if (MODE != 1) pdl_wait();     // the shell launch beside this one
 }
 
 // ----------------------------------------------------------------- host --
@@ -701,16 +712,6 @@ static int tma_mode(const FitParams<T>& p) {
   for (int f = 0; f < 4; f++)
     if (p.pec_face[f] != 0) return 0;
   return (p.pec_face[4] == 0 && p.pec_face[5] == 0) ? 1 : 2;
-}
-
-// The TMA kernel on row groups needs a shell pair after it unless every face
-// is PEC-masked; on small grids the two passes are then as fast.  Measured on
-// B200, two-pass / TMA (us a step): 33x37x65 FP64 periodic 29.0 / 29.1, open
-// ends 29.2 / 28.6, 45x45x110 FP64 periodic 43.6 / 41.4; 45x45x110 FP32 open
-// 30.4 / 32.2, 61x61x130 FP32 periodic 45.2 / 43.4, open 43.7 / 34.2.
-template <typename T>
-bool tma_preferred(const FitParams<T>& p) {
-  return row_group(p) == 1 || tma_mode(p) == 1 || p.N >= (sizeof(T) == 8 ? 100000 : 400000);
 }
 
 // True when the TMA kernel can run this grid: 16-byte aligned buffers, dims
@@ -775,18 +776,19 @@ static cudaError_t launch_tma_variant(const FitParams<T>& p, long long step, cud
   if (KC <= 0)
     KC = tma_auto_kc((long long)gx * gy, planes, (long long)occ->sms * occ->per_sm);
   const int gz = (planes + KC - 1) / KC;
+  // shell (MODE 2: the four boundary planes only) from the old state, the tiles
+  // beside it
+  if (MODE != 1 && (e = launch_shell_step<T>(p, step, st, MODE == 2)) != cudaSuccess) return e;
+  const auto kern = k_tma<T, SM, JM, MODE, DESC, GRP, TW>;
+  const dim3 grid(gx, gy, gz);
+  const int smem = TmaLayout<T, (MODE != 0), GRP, TW>::bytes, lg = group == 4 ? 2 : group - 1;
   timer_begin(st);
-  k_tma<T, SM, JM, MODE, DESC, GRP, TW><<<dim3(gx, gy, gz), kTmaThreads,
-                                          TmaLayout<T, (MODE != 0), GRP, TW>::bytes, st>>>(
-      p, maps, step, KC, group == 4 ? 2 : group - 1);
+  if (MODE == 1)
+    kern<<<grid, kTmaThreads, smem, st>>>(p, maps, step, KC, lg);
+  else
+    e = launch_beside(kern, grid, kTmaThreads, smem, st, p, maps, step, KC, lg);
   timer_end(st);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (MODE == 1) return cudaSuccess;
-  // shell (MODE 2: the four boundary planes only): H from the old state, then
-  // E from the new H (the H the shell E rows read is in H_out once k_tma is
-  // done)
-  return launch_shell_pair<T>(p, step, st, MODE == 2);
+  return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 // Whether 32x16 tiles take less time than 64x8 ones: the lanes of the tiles
@@ -845,19 +847,8 @@ cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, i
   return cudaErrorInvalidValue;
 }
 
-// Launches per step of the TMA schedule for these parameters: 1 (every face
-// PEC-masked) or 3 (TMA kernel + two shell launches).
-template <typename T>
-int tma_launches_per_step(const FitParams<T>& p) {
-  return tma_mode(p) == 1 ? 1 : 3;
-}
-
-template bool tma_preferred<double>(const FitParams<double>&);
-template bool tma_preferred<float>(const FitParams<float>&);
 template bool tma_pitch<double>(const FitParams<double>&);
 template bool tma_pitch<float>(const FitParams<float>&);
-template int tma_launches_per_step<double>(const FitParams<double>&);
-template int tma_launches_per_step<float>(const FitParams<float>&);
 template bool tma_supported<double>(const FitParams<double>&);
 template bool tma_supported<float>(const FitParams<float>&);
 template cudaError_t launch_tma<double>(const FitParams<double>&, long long, cudaStream_t, int,

@@ -16,6 +16,7 @@ k_tma_comp(FitParams<double> p, CompState cs, const __grid_constant__ CompMaps m
   extern __shared__ __align__(128) unsigned char sm_raw[];
   comp_tile<IdT, SIG, MODE, CT ? 1 : 0, false, TW>(p, cs, maps, step, KC, blockIdx.x,
                                                    blockIdx.y, blockIdx.z, CT, sm_raw);
+  if (MODE != 1) pdl_wait();     // the H shell launch beside this one
 }
 
 // id width x J mode x face mode x compensation words by TMA x tile width
@@ -133,9 +134,12 @@ cudaError_t launch_tma_comp(const wk_fit_desc* d, const FitParams<double>& p, in
                      (long long)g_comp_sms[slot][dev] * g_comp_per_sm[slot][dev]);
   const int gz = (planes + KC - 1) / KC;
   timer_begin(st);
-  kern<<<dim3(gx, gy, gz), cThreads, smem, st>>>(p, cs, maps, step, KC);
+  if (mode == 1)
+    kern<<<dim3(gx, gy, gz), cThreads, smem, st>>>(p, cs, maps, step, KC);
+  else
+    e = launch_beside(kern, dim3(gx, gy, gz), cThreads, smem, st, p, cs, maps, step, KC);
   timer_end(st);
-  return cudaGetLastError();
+  return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace wk
