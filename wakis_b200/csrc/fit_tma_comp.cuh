@@ -209,7 +209,7 @@ __device__ __forceinline__ float row_value(double dt, double f, double g) {
 // conductive J mode) rather than zero; CT: the compensation words of plane k
 // arrive by TMA with H(k) (row pitch Nx % 8 == 0) instead of per-thread
 // loads issued one plane ahead.  MODE 0: interior cells, the shell
-// follows in separate launches.  MODE 1: every face carries the PEC column
+// in launches of its own (H beside this one, E after it).  MODE 1: every face carries the PEC column
 // mask (no PMC); the tiles cover the whole grid and the cells on or next to
 // a face use the same rows with the masked entries set to zero (E entries
 // tangential to a face they lie on enter no H row; E rows tangential to
