@@ -293,24 +293,26 @@ k_shell_step(FitParams<T> p, long long step, int total) {
   const T* const hx = p.H_in;
   const T* const hy = hx + p.N;
   const T* const hz = hy + p.N;
-  auto ld = [&](const T* f, int q) { return q < N ? __ldg(f + q) : T(0); };
+  auto ld = [&](const T* f, int q, int off) {
+    return inside_after(q, off, N) ? __ldg(f + q + off) : T(0);
+  };
   const int id = load_id(p.mat_id, p.id_bytes, n);
   const int idx_ = load_id(p.mat_id, p.id_bytes, mx), idy = load_id(p.mat_id, p.id_bytes, my),
             idz = load_id(p.mat_id, p.id_bytes, mz);
   const T ex0 = __ldg(ex + n), ey0 = __ldg(ey + n), ez0 = __ldg(ez + n);
-  const T ey1 = ld(ey, n + 1), ez1 = ld(ez, n + 1);
-  const T ex2 = ld(ex, n + Nx), ez2 = ld(ez, n + Nx);
-  const T ex3 = ld(ex, n + NxNy), ey3 = ld(ey, n + NxNy);
+  const T ey1 = ld(ey, n, 1), ez1 = ld(ez, n, 1);
+  const T ex2 = ld(ex, n, Nx), ez2 = ld(ez, n, Nx);
+  const T ex3 = ld(ex, n, NxNy), ey3 = ld(ey, n, NxNy);
   T h0 = __ldg(hx + n), h1 = __ldg(hy + n), h2 = __ldg(hz + n);
   // x neighbour: rows y, z; y neighbour: rows x, z; z neighbour: rows x, y
   const T xex = __ldg(ex + mx), xey = __ldg(ey + mx), xez = __ldg(ez + mx);
-  const T xex2 = ld(ex, mx + Nx), xex3 = ld(ex, mx + NxNy);
+  const T xex2 = ld(ex, mx, Nx), xex3 = ld(ex, mx, NxNy);
   T xhx = T(0), xhy = __ldg(hy + mx), xhz = __ldg(hz + mx);
   const T yex = __ldg(ex + my), yey = __ldg(ey + my), yez = __ldg(ez + my);
-  const T yey1 = ld(ey, my + 1), yey3 = ld(ey, my + NxNy);
+  const T yey1 = ld(ey, my, 1), yey3 = ld(ey, my, NxNy);
   T yhx = __ldg(hx + my), yhy = T(0), yhz = __ldg(hz + my);
   const T zex = __ldg(ex + mz), zey = __ldg(ey + mz), zez = __ldg(ez + mz);
-  const T zez1 = ld(ez, mz + 1), zez2 = ld(ez, mz + Nx);
+  const T zez1 = ld(ez, mz, 1), zez2 = ld(ez, mz, Nx);
   T zhx = __ldg(hx + mz), zhy = __ldg(hy + mz), zhz = T(0);
   const bool desc = p.h_desc != 0;
   const T z = T(0);

@@ -134,6 +134,11 @@ inline long long shell_cells(int Nx, int Ny, int Nz, bool planes_only) {
   const long long planes = 4LL * Nx * Ny;
   return planes_only ? planes : planes + 4LL * (Nz - 4) * (Nx + Ny - 4);
 }
+// Whether cell n + off lies in a grid of N cells (0 <= n < N, 0 <= off <= N):
+// the sum itself can pass 2^31 on the top planes of the largest grids.
+__host__ __device__ __forceinline__ bool inside_after(int n, int off, int N) {
+  return n < N - off;
+}
 __device__ __forceinline__ Cell shell_cell(int idx, int Nx, int Ny, int Nz) {
   Cell c;
   const int NxNy = Nx * Ny;
