@@ -1,0 +1,62 @@
+"""Calls at the edges of a kernel's or a rule's range, each against the general
+path or the definition."""
+
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+PEC = (["pec"] * 3, ["pec"] * 3)
+OPEN = (["pec", "pec", "abc"], ["pec", "pec", "abc"])
+
+
+def _ptr(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _solver(shape, bcs=PEC, dtype=np.float64, sigma=10.0, **kw):
+    import wakis_b200 as wb
+    g = wb.GridFIT3D(-0.03, 0.031, -0.02, 0.022, -0.04, 0.043, *shape, verbose=0)
+    m = np.zeros(shape, bool)
+    m[2:shape[0] // 2, 3:shape[1] // 2, 1:shape[2] // 2] = True
+    g.add_solid("a", m, [4.0, 1.0, sigma])
+    return wb.SolverFIT3D(g, bc_low=bcs[0], bc_high=bcs[1], dtype=dtype, bg=[1.0, 1.0],
+                          use_stl=True, use_sibc=False, verbose=0, **kw)
+
+
+def _random_state(s, e=True, seed=7):
+    rng = np.random.default_rng(seed)
+    s._first_step()
+    if e:
+        s.E.fromarray(300 * rng.standard_normal(3 * s.N))
+    s.H.fromarray(rng.standard_normal(3 * s.N))
+
+
+def _equal(a, b):
+    return torch.equal(a.E.array, b.E.array) and torch.equal(a.H.array, b.H.array)
+
+
+@pytest.mark.parametrize("dtype,shape", [(np.float32, (71, 21, 13)), (np.float32, (70, 33, 11)),
+                                         (np.float32, (33, 35, 19)), (np.float64, (71, 21, 13)),
+                                         (np.float64, (33, 35, 19))])
+@pytest.mark.parametrize("tile", [(8, 1), (8, 2), (8, 5), (16, 3), (16, 64)])
+def test_last_partial_row_group(dtype, shape, tile):
+    """Closed grids whose 3 Ny Nz rows are no multiple of the group: the rows
+    past the last whole group, filled in by hand on the top plane, wherever
+    the chunks of planes end."""
+    sol = []
+    for kernel in ("auto", "twopass"):
+        s = _solver(shape, dtype=dtype)
+        s.kernel, s.tile, s.steps_per_launch = kernel, tile, 1
+        _random_state(s)
+        s._advance(6, 0)
+        s.check_status()
+        sol.append(s)
+    assert _equal(*sol)

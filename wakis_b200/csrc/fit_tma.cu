@@ -440,7 +440,12 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
         if (pl == pstart) patch(pl, Eb + se * 3 * SE, etab + se * 3 * S::BY, S::BY, S::TX + 2, p.E_in);
         patch(pl + 1, Eb + se2 * 3 * SE, etab + se2 * 3 * S::BY, S::BY, S::TX + 2, p.E_in);
       }
+      // H's table was written by warp 8 (LATE: since the last block barrier)
+      if (pl == Nz - 1) asm volatile("bar.sync 1, 64;" ::: "memory");
       patch(pl, Hb + sh * 3 * SH, htab + sh * 3 * S::HBY, S::HBY, S::TX + 1, p.H_in);
+    } else if (GRP && issue_wh && pl == Nz - 1) {
+      __syncwarp();
+      asm volatile("bar.sync 1, 64;" ::: "memory");    // warps 8 and 9
     }
     ok = __syncthreads_and(got);
     if (!ok) break;
