@@ -60,3 +60,25 @@ def test_last_partial_row_group(dtype, shape, tile):
         s.check_status()
         sol.append(s)
     assert _equal(*sol)
+
+
+@pytest.mark.parametrize("dtype,shape", [(np.float64, (33, 24, 20)), (np.float64, (9, 8, 5)),
+                                         (np.float32, (34, 24, 20)), (np.float32, (33, 17, 21)),
+                                         (np.float64, (32, 24, 20)), (np.float32, (32, 17, 21))])
+def test_two_steps_per_launch_on_any_row_length(dtype, shape):
+    """steps_per_launch = 2 on closed, clean grids: rows that are no multiple
+    of 16 bytes take one step per launch, the others pairs; the fields are the
+    two-pass schedule's either way."""
+    from wakis_b200.sources import Beam
+    sol = []
+    for kernel, spl in (("auto", 2), ("twopass", 1)):
+        s = _solver(shape, dtype=dtype)
+        s.kernel, s.steps_per_launch = kernel, spl
+        bp = Beam(q=1e-9, sigmaz=0.005).params(s)
+        s._advance(10, 0, beam=bp)
+        s._advance(7, 10, beam=bp)
+        s.check_status()
+        sol.append(s)
+    a, b = sol
+    assert a._faces_clean and np.abs(a.E.numpy()).max() > 0
+    assert _equal(a, b)

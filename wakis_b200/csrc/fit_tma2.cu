@@ -476,12 +476,13 @@ static bool encode2(CUtensorMap* map, const T* base, int Nx, int Ny, int Nz, int
 }
 
 // True when two steps of these parameters can run as one k_tma2 launch:
-// the TMA conditions, every face PEC-masked (no PMC), clean faces, J = 0
+// the TMA conditions with a row and component pitch of 16 bytes (its boxes are
+// of single rows), every face PEC-masked (no PMC), clean faces, J = 0
 // without conductivity or J = sigma*E with it (no stored J); the source
 // line (fused beam or line buffer) is applied in both steps.
 template <typename T>
 bool tma2_supported(const FitParams<T>& p) {
-  if (!tma_supported<T>(p)) return false;
+  if (!tma_supported<T>(p) || !tma_pitch<T>(p)) return false;
   if (!p.has_pec || p.has_pmc) return false;
   for (int f = 0; f < 6; f++)
     if (p.pec_face[f] != 0) return false;
