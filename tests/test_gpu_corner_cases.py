@@ -82,3 +82,26 @@ def test_two_steps_per_launch_on_any_row_length(dtype, shape):
     a, b = sol
     assert a._faces_clean and np.abs(a.E.numpy()).max() > 0
     assert _equal(a, b)
+
+
+@pytest.mark.parametrize("ns,n_win", [(1, 1), (33, 9), (64, 3)])
+@pytest.mark.parametrize("carry", [0, 1])
+@pytest.mark.parametrize("q", [1e3, -1e3])
+def test_wake_potential_of_no_z_cells_is_the_empty_sum(ns, n_win, carry, q):
+    """nz = 0: every sample of every window is written, as 0 / q."""
+    from wakis_b200 import _native
+    f = lambda n: torch.ones(n, dtype=torch.float64, device="cuda")
+    hist, z, s = f(n_win * 2 * 8), f(1), f(ns)
+    win = torch.arange(n_win, dtype=torch.int32, device="cuda")
+    order = torch.arange(8, dtype=torch.int64, device="cuda")
+    WP = torch.full((n_win, ns), float("nan"), dtype=torch.float64, device="cuda")
+    _native.check(_native.lib().wk_wake_potential(
+        _ptr(hist), _native.WK_F64, 8, 2, _ptr(win), n_win, carry, _ptr(z), _ptr(z), 0, 0, _ptr(s),
+        ns, _ptr(order), 8, 3e8, 0.0, 1.0, 0.0, 0.0, 1e-12, q, 0, _ptr(WP), _stream()),
+        "wk_wake_potential")
+    ref = np.empty((n_win, ns))
+    acc = np.zeros(ns)
+    for w in range(n_win):
+        ref[w] = acc = (acc if carry else np.zeros(ns)) / q
+    got = WP.cpu().numpy()
+    assert np.array_equal(got, ref) and np.array_equal(np.signbit(got), np.signbit(ref))

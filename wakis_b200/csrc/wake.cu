@@ -69,6 +69,14 @@ k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
   const bool on = n < g.ns;
   const int terms = g.n_win * g.nz;
   const int chunks = (terms + kWakeChunk - 1) / kWakeChunk;
+  if (terms == 0) {                          // empty sums
+    double acc = 0.0;
+    for (int w = 0; w < g.n_win && warp == 0 && on; w++) {
+      acc = __ddiv_rn(g.carry ? acc : 0.0, g.qnorm);
+      WP3d[(long long)w * g.ns + n] = acc;
+    }
+    return;
+  }
   if (warp < kWakeProd) {
     const double sn = s[on ? n : g.ns - 1];
     // entry and coefficient of term q (window q / nz, z index q % nz): the
