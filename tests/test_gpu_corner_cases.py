@@ -105,3 +105,36 @@ def test_wake_potential_of_no_z_cells_is_the_empty_sum(ns, n_win, carry, q):
         ref[w] = acc = (acc if carry else np.zeros(ns)) / q
     got = WP.cpu().numpy()
     assert np.array_equal(got, ref) and np.array_equal(np.signbit(got), np.signbit(ref))
+
+
+@pytest.mark.parametrize("length,N,at", [(300, 700, 3), (300, 701, 257), (1000, 4001, 999), (40, 64, 0)])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 1.7e308])
+def test_dft_bins_of_infinite_signals(length, N, at, value):
+    """One infinite entry (or ones whose sum overflows) gives infinite parts
+    where the term-by-term sum is infinite and NaN only where that sum is NaN;
+    the signal beside it is not affected."""
+    from wakis_b200 import _native
+    rng = np.random.default_rng(at)
+    x = rng.standard_normal((2, length))
+    x[0, at] = value
+    if np.isfinite(value):
+        x[0, :] = value                       # bin 0 overflows
+    nb = 6
+    out = torch.empty((2, nb, 2), dtype=torch.float64, device="cuda")
+    t = torch.as_tensor(x, device="cuda")
+    _native.check(_native.lib().wk_dft_bins(_ptr(t), 2, length, N, nb, _ptr(out), _stream()),
+                  "wk_dft_bins")
+    got = out.cpu().numpy()
+    assert np.isfinite(got[1]).all()
+    if np.isfinite(value):
+        assert got[0, 0, 0] == np.inf and got[0, 0, 1] == 0.0
+        return
+    for m in range(nb):
+        # exact quarter turns decide where an infinite entry meets a zero
+        r = (m * at) % N
+        turn = 2 * np.pi * r / N
+        c = 0.0 if 4 * r in (N, 3 * N) else np.cos(turn)
+        s = 0.0 if 2 * r in (0, N) else np.sin(turn)
+        for part, f in ((0, c), (1, -s)):
+            want = value * f if f != 0 and not np.isnan(value) else np.nan
+            assert np.array_equal(got[0, m, part], want, equal_nan=True), (m, part)
