@@ -138,3 +138,32 @@ def test_dft_bins_of_infinite_signals(length, N, at, value):
         for part, f in ((0, c), (1, -s)):
             want = value * f if f != 0 and not np.isnan(value) else np.nan
             assert np.array_equal(got[0, m, part], want, equal_nan=True), (m, part)
+
+
+@pytest.mark.parametrize("nz", [1, 5])
+def test_wake_potential_of_a_history_past_int_columns(nz):
+    """More than 2^31 columns (FP32, 8.6 GB a row): the entries of the last
+    ones are the ones read."""
+    from wakis_b200 import _native
+    nt, rows, ns, dt = 2 ** 31 + 9, 1, 8 - nz + 1, 1e-12
+    hist = torch.empty(rows * nt * (1 if nz == 1 else 5), dtype=torch.float32, device="cuda")
+    rows = hist.numel() // nt
+    order = torch.arange(nt - 8, nt, dtype=torch.int64, device="cuda")
+    rng = np.random.default_rng(1)
+    vals = rng.standard_normal((rows, 8)).astype(np.float32)
+    for r in range(rows):
+        hist[r * nt + nt - 8:(r + 1) * nt] = torch.as_tensor(vals[r], device="cuda")
+        hist[r * nt:r * nt + 8] = float("nan")
+    v = 1.0 / dt                              # column = z + s in units of one
+    f = lambda a: torch.as_tensor(np.asarray(a, dtype=np.float64), device="cuda")
+    z, dz, s = f(np.arange(nz) + 0.0), f(np.ones(nz)), f(np.arange(ns) + 0.25)
+    WP = torch.full((1, ns), float("nan"), dtype=torch.float64, device="cuda")
+    win = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _native.check(_native.lib().wk_wake_potential(
+        _ptr(hist), _native.WK_F32, nt, rows, _ptr(win), 1, 0, _ptr(z), _ptr(dz), nz, 0, _ptr(s),
+        ns, _ptr(order), 8, v, 0.0, 1.0, 0.0, 0.0, dt, 1.0, 0, _ptr(WP), _stream()),
+        "wk_wake_potential")
+    ref = np.zeros(ns)
+    for k in range(nz):
+        ref += vals[k, np.arange(ns) + k].astype(np.float64)
+    assert np.array_equal(WP.cpu().numpy()[0], ref)

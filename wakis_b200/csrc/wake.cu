@@ -25,7 +25,8 @@ struct WakeArgs {
   long long hist_nt, nt;
   double v, zmin_v, zmax_v, t0, ti, dt, qnorm;
 };
-__device__ __forceinline__ int wake_column(const WakeArgs& g, const double* __restrict__ z,
+template <typename Idx>
+__device__ __forceinline__ Idx wake_column(const WakeArgs& g, const double* __restrict__ z,
                                            const long long* __restrict__ key_order, double sn,
                                            int k) {
   const int kr = g.counter_moving ? g.nz - 1 - k : k;
@@ -39,7 +40,7 @@ __device__ __forceinline__ int wake_column(const WakeArgs& g, const double* __re
   if (it < 0) it += g.nt;                          // negative index wraps as in numpy
   if (it < 0) return -1;
   const long long t = __ldg(key_order + it);
-  return t >= 0 && t < g.hist_nt ? (int)t : -1;    // -1: no such history column
+  return t >= 0 && t < g.hist_nt ? (Idx)t : -1;    // -1: no such history column
 }
 
 // One block per 32 samples.  The sum over z is sequential, window after window
@@ -50,13 +51,14 @@ __device__ __forceinline__ int wake_column(const WakeArgs& g, const double* __re
 // of a row for the lanes of a warp) being read while the chunk before is
 // formed.  A term that does not exist is -0, which leaves any sum as it is.
 // The columns, two divisions each, are formed once per (sample, z) and kept in
-// shared memory for the other windows when they fit (COLS).
+// shared memory for the other windows when they fit (COLS).  Idx: long long
+// where a column or a term's number does not fit an int.
 // Bound by the chain and the history's read.  On B200, 9 windows of nz = 400,
 // ns = 11700, FP64: 272 us (345 MB), nz = 120, ns = 4700 55 us; 2632 with one thread per sample
 // that formed the column of every term and waited for its entry, 1158 with one
 // warp per block doing both parts; 4 terms per warp and chunk 257 and 85 us.
 constexpr int kWakeProd = 8, kWakeEach = 2, kWakeChunk = kWakeProd * kWakeEach;
-template <typename H, bool COLS>
+template <typename H, bool COLS, typename Idx>
 __global__ void __launch_bounds__((kWakeProd + 1) * 32)
 k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
                  const double* __restrict__ z, const double* __restrict__ dz,
@@ -67,8 +69,8 @@ k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
   int* cols = reinterpret_cast<int*>(term + 2 * kWakeChunk * 32);   // [nz][32] (COLS)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = blockIdx.x * 32 + lane;
   const bool on = n < g.ns;
-  const int terms = g.n_win * g.nz;
-  const int chunks = (terms + kWakeChunk - 1) / kWakeChunk;
+  const Idx terms = (Idx)g.n_win * g.nz;
+  const Idx chunks = (terms + kWakeChunk - 1) / kWakeChunk;
   if (terms == 0) {                          // empty sums
     double acc = 0.0;
     for (int w = 0; w < g.n_win && warp == 0 && on; w++) {
@@ -87,15 +89,15 @@ k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
       H entry[kWakeEach];
       bool have[kWakeEach];
     };
-    auto read = [&](int chunk, Terms& v) {
-      const int q0 = chunk * kWakeChunk + warp * kWakeEach;
-      int w = q0 / g.nz, k = q0 - w * g.nz;
+    auto read = [&](Idx chunk, Terms& v) {
+      const Idx q0 = chunk * kWakeChunk + warp * kWakeEach;
+      int w = (int)(q0 / g.nz), k = (int)(q0 - (Idx)w * g.nz);
 #pragma unroll
       for (int u = 0; u < kWakeEach; u++) {
         v.have[u] = false;
         if (q0 + u < terms) {
-          const int t = COLS && w > 0 ? cols[k * 32 + lane]
-                                      : (on ? wake_column(g, z, key_order, sn, k) : -1);
+          const Idx t = COLS && w > 0 ? cols[k * 32 + lane]
+                                      : (on ? wake_column<Idx>(g, z, key_order, sn, k) : -1);
           if (COLS && w == 0) cols[k * 32 + lane] = t;
           const int kz = (g.counter_moving ? g.nz - 1 - k : k) + g.k_off;
           const double c = __ldg(dz + k);
@@ -108,7 +110,7 @@ k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
         if (++k == g.nz) { k = 0; w++; }
       }
     };
-    auto put = [&](int chunk, const Terms& v) {
+    auto put = [&](Idx chunk, const Terms& v) {
       double* out = term + (chunk & 1) * kWakeChunk * 32 + warp * kWakeEach * 32 + lane;
 #pragma unroll
       for (int u = 0; u < kWakeEach; u++)
@@ -119,7 +121,7 @@ k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
     Terms va, vb;
     read(0, va);
     read(1, vb);
-    for (int c = 0; c < chunks; c += 2) {
+    for (Idx c = 0; c < chunks; c += 2) {
       put(c, va);
       read(c + 2, va);
       if (c + 1 < chunks) {
@@ -130,7 +132,7 @@ k_wake_potential(const H* __restrict__ hist, const int* __restrict__ win_map,
   } else {
     double acc = 0.0;
     int w = 0, k = 0;
-    for (int c = 0; c < chunks; c++) {
+    for (Idx c = 0; c < chunks; c++) {
       __syncthreads();
       const double* in = term + (c & 1) * kWakeChunk * 32 + lane;
       if (k + kWakeChunk < g.nz) {           // no window ends in this chunk
@@ -168,16 +170,20 @@ cudaError_t launch_wake_potential(const H* hist, const int* win_map, const doubl
                                   const WakeArgs& g, double* WP3d, cudaStream_t st) {
   const int blocks = (g.ns + 31) / 32;
   const int threads = (kWakeProd + 1) * 32;
-  if (g.nz >= kWakeColsMin && g.nz <= kWakeColsMax) {
-    cudaError_t e = cudaFuncSetAttribute(k_wake_potential<H, true>,
+  const long long most = 0x7fffffffLL - 4 * kWakeChunk;
+  if (g.hist_nt > most || (long long)g.n_win * g.nz > most) {
+    k_wake_potential<H, false, long long><<<blocks, threads, kWakeTermBytes, st>>>(
+        hist, win_map, z, dz, s, key_order, g, WP3d);
+  } else if (g.nz >= kWakeColsMin && g.nz <= kWakeColsMax) {
+    cudaError_t e = cudaFuncSetAttribute(k_wake_potential<H, true, int>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kWakeTermBytes + kWakeColsMax * 128);
     if (e != cudaSuccess) return e;
-    k_wake_potential<H, true><<<blocks, threads, kWakeTermBytes + g.nz * 128, st>>>(
+    k_wake_potential<H, true, int><<<blocks, threads, kWakeTermBytes + g.nz * 128, st>>>(
         hist, win_map, z, dz, s, key_order, g, WP3d);
   } else {
-    k_wake_potential<H, false><<<blocks, threads, kWakeTermBytes, st>>>(hist, win_map, z, dz, s,
-                                                                        key_order, g, WP3d);
+    k_wake_potential<H, false, int><<<blocks, threads, kWakeTermBytes, st>>>(
+        hist, win_map, z, dz, s, key_order, g, WP3d);
   }
   return cudaGetLastError();
 }
@@ -635,8 +641,6 @@ extern "C" int wk_wake_potential(const void* hist, int hist_dtype, long long his
                    ns, nz, n_win, nt);
   if (ns == 0) return WK_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (hist_nt > 0x7fffffffLL)
-    return wk_fail(WK_E_RANGE, "wk_wake_potential: history of %lld columns", hist_nt);
   WakeArgs g;
   g.nz = nz; g.k_off = k_off; g.ns = ns; g.counter_moving = counter_moving;
   g.n_win = n_win; g.carry = carry; g.Nzh = Nzh;
