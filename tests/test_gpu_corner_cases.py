@@ -167,3 +167,21 @@ def test_wake_potential_of_a_history_past_int_columns(nz):
     for k in range(nz):
         ref += vals[k, np.arange(ns) + k].astype(np.float64)
     assert np.array_equal(WP.cpu().numpy()[0], ref)
+
+
+@pytest.mark.parametrize("ns", [65535, 65536, 65537, 131073, 200003])
+def test_transverse_prefix_sums_of_long_axes(ns):
+    """Axes on both sides of 128 * 2^9 samples, where another kernel takes them:
+    numpy's sums value for value."""
+    from wakis_b200 import _native
+    rng = np.random.default_rng(ns)
+    WP = rng.standard_normal((9, ns))
+    t = torch.as_tensor(WP, device="cuda")
+    wx, wy = (torch.empty(ns, dtype=torch.float64, device="cuda") for _ in range(2))
+    ds, dx, dy = 1e-3, 2e-3, 3e-3
+    _native.check(_native.lib().wk_trans_wake(_ptr(t), ns, ds, dx, dy, _ptr(wx), _ptr(wy), _stream()),
+                  "wk_trans_wake")
+    wx, wy = wx.cpu().numpy(), wy.cpu().numpy()
+    for n in sorted(set(rng.integers(0, ns, 100).tolist()) | {0, 1, 129, 65534, ns - 1}):
+        i = {w: np.sum(WP[w, 0:n]) * ds for w in (7, 1, 5, 3)}
+        assert wx[n] == -(i[7] - i[1]) / dx and wy[n] == -(i[5] - i[3]) / dy

@@ -366,6 +366,24 @@ k_trans_wake(const double* __restrict__ WP3d, int ns, double ds, double dxsum, d
   }
 }
 
+// Axes longer than the tree of calls reaches (128 * 2^9 samples): one thread per
+// sample.  A warp per sample would walk the long nodes lane by lane: 90000
+// samples 31.3 ms, so 11.3; with a deeper tree of calls (255 registers) 15.5,
+// 200000 samples 78 and 35.  At 65536 the warps take 4.7 ms and the threads 6.5.
+constexpr int kTransWarpMax = 65536;
+__global__ void k_trans_wake_long(const double* __restrict__ WP3d, int ns, double ds, double dxsum,
+                                  double dysum, double* __restrict__ WPx,
+                                  double* __restrict__ WPy) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= ns) return;
+  const double ixp = __dmul_rn(pw_sum(WP3d + 7LL * ns, n), ds);
+  const double ixm = __dmul_rn(pw_sum(WP3d + 1LL * ns, n), ds);
+  const double iyp = __dmul_rn(pw_sum(WP3d + 5LL * ns, n), ds);
+  const double iym = __dmul_rn(pw_sum(WP3d + 3LL * ns, n), ds);
+  WPx[n] = __ddiv_rn(-__dsub_rn(ixp, ixm), dxsum);
+  WPy[n] = __ddiv_rn(-__dsub_rn(iyp, iym), dysum);
+}
+
 // ------------------------------------------------------------- streaming --
 // The s sample index n and z index k of the sum for WP(s_n) read step
 // it(n, k) = (long)(ts/dt) (same rounded expression as k_wake_potential).
@@ -661,7 +679,12 @@ extern "C" int wk_trans_wake(const double* WP3d, int ns, double ds, double dxsum
   if (ns < 0) return wk_fail(WK_E_RANGE, "wk_trans_wake: ns %d", ns);
   if (ns == 0) return WK_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  k_trans_wake<<<(ns + kTransWarps - 1) / kTransWarps, kTransWarps * 32, 0, st>>>(WP3d, ns, ds, dxsum, dysum, WPx, WPy);
+  if (ns > kTransWarpMax)
+    k_trans_wake_long<<<(unsigned)((ns + 127LL) / 128), 128, 0, st>>>(WP3d, ns, ds, dxsum, dysum,
+                                                                      WPx, WPy);
+  else
+    k_trans_wake<<<(ns + kTransWarps - 1) / kTransWarps, kTransWarps * 32, 0, st>>>(
+        WP3d, ns, ds, dxsum, dysum, WPx, WPy);
   return wk_check_launch("wk_trans_wake");
 }
 
