@@ -83,3 +83,37 @@ def test_a_replaced_step_is_run(name, how, monkeypatch):
     ref = _stepwise()
     for n in NAMES:
         assert np.allclose(getattr(w, n), getattr(ref, n), rtol=1e-14, atol=0), n
+
+
+@pytest.mark.parametrize("fails,kept", [("_trans", ["WP", "WP_3d"]),
+                                        ("_dft", ["WP", "WP_3d", "WPx", "WPy"]), ("_wp", [])])
+def test_a_step_that_fails_leaves_the_results_before_it(fails, kept):
+    """A second solve whose transverse integration or DFT raises (a range of
+    frequencies without bins, say): the error, the new results of the steps
+    before it, the earlier ones of the steps after it, the line density as
+    given."""
+    w, WP, WPxy = _wake()
+    for n in NAMES:
+        setattr(w, n, "earlier")
+
+    def bad(self, *a, **k):
+        raise ZeroDivisionError("no bins")
+
+    setattr(w, fails, types.MethodType(bad, w))
+    with pytest.raises(ZeroDivisionError):
+        w.solve()
+    ref = _stepwise()
+    for n in NAMES:
+        if n in kept:
+            assert np.array_equal(getattr(w, n), getattr(ref, n)), n
+        else:
+            assert getattr(w, n) == "earlier", n
+    assert (w.lambdas is None) == (fails != "_dft")
+
+
+def test_a_line_density_that_cannot_be_scaled_is_refused():
+    w, WP, WPxy = _wake()
+    w.lambdas = [0.0] * NS
+    with pytest.raises(TypeError):
+        w.solve()
+    assert np.array_equal(w.WPx, WPxy[0]) and w.Z is None

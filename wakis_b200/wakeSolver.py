@@ -223,33 +223,39 @@ class WakeSolver:
         kernels queued behind one another, one upload of the line density, one
         set of DFT bins for all planes and one copy of the results to the host
         (a copy after each took 0.7 of 1.5 ms for 400 x 12000 samples, in which
-        the device waited).  False, with nothing done, where the line density
-        is not known before the wake potential or where one of the steps is
-        not this class's own (a subclass or a program replaced it)."""
+        the device waited).  False, the results as they were, where the line
+        density is not known before the wake potential, where one of the steps
+        is not this class's own (a subclass or a program replaced it) or where
+        a part of it fails."""
         stream = getattr(self, "_stream", None)
         if self._hist_1d or (self._hist is None and stream is None):
             return False
         if not all(getattr(getattr(self, f.__name__), "__func__", None) is f for f in self._STEPS):
             return False
+        given = self.lambdas
+        try:
+            done = self._solve_queued(stream)
+        except Exception:
+            done = False       # the steps raise it, after the results before it are set
+        if not done:
+            self.lambdas = given
+        return done
+
+    def _solve_queued(self, stream):
         s = self._axis()[-1] if stream is None else self.s
         if len(s) < 3 or len(s) > self.TRANS_PAIRWISE_MAX:
             return False
-        given = self.lambdas
-        if given is None:
+        if self.lambdas is None:
             if self.chargedist is not None:
                 return False
             self.s = s
             self.calc_lambdas_analytic()
-        lambdas = np.asarray(self.lambdas)
+        lambdas = np.asarray(self.lambdas * self.v)
         if lambdas.shape != s.shape or np.iscomplexobj(lambdas):
             return False
         dev = (self._hist if stream is None else stream["acc"]).device
-        lam, = self._upload(dev, lambdas * self.v)
-        try:
-            WP3d = self._wp(9, carry=True)
-        except Exception:
-            self.lambdas = given
-            raise
+        lam, = self._upload(dev, lambdas)
+        WP3d = self._wp(9, carry=True)
         self._WP3d_dev, self._WP_dev = WP3d, WP3d[4]
         WPxy = self._trans(WP3d)
         self._WPx_dev, self._WPy_dev = WPxy[0], WPxy[1]
