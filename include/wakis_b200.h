@@ -399,8 +399,9 @@ int wk_fit_step(const wk_fit_desc* d, int n_steps, long long step0, void* stream
 /*
  * 1 when a wk_fit_step call of n_steps steps on this descriptor runs them all
  * in one launch (a small grid with `sync` words and the automatic kernel), 0
- * when not, or when the descriptor is not valid.  No counterpart in the
- * reference.
+ * when not, or when the descriptor is not valid.  In a context that is given
+ * a part of the device's SMs such a call may run step by step all the same.  No
+ * counterpart in the reference.
  */
 int wk_fit_one_launch(const wk_fit_desc* d, int n_steps);
 

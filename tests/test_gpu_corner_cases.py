@@ -185,3 +185,47 @@ def test_transverse_prefix_sums_of_long_axes(ns):
     for n in sorted(set(rng.integers(0, ns, 100).tolist()) | {0, 1, 129, 65534, ns - 1}):
         i = {w: np.sum(WP[w, 0:n]) * ds for w in (7, 1, 5, 3)}
         assert wx[n] == -(i[7] - i[1]) / dx and wy[n] == -(i[5] - i[3]) / dy
+
+
+@pytest.fixture
+def few_sms():
+    """A stream of a context that has a part of the device's SMs."""
+    drv = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        if int(r[0]) != 0:
+            pytest.skip(f"no partition of the SMs here ({r[0]})")
+        return r[1] if len(r) == 2 else r[1:]
+
+    torch.zeros(1, device="cuda")
+    dev = ok(drv.cuDeviceGet(torch.cuda.current_device()))
+    sm = ok(drv.cuDeviceGetDevResource(dev, drv.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    parts, _, _ = ok(drv.cuDevSmResourceSplitByCount(1, sm, 0, 16))
+    desc = ok(drv.cuDevResourceGenerateDesc(parts, 1))
+    ctx = ok(drv.cuGreenCtxCreate(desc, dev, drv.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(drv.cuGreenCtxStreamCreate(
+        ctx, drv.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    yield torch.cuda.ExternalStream(int(stream))
+    torch.cuda.synchronize()
+    drv.cuStreamDestroy(stream)
+    drv.cuGreenCtxDestroy(ctx)
+
+
+@pytest.mark.parametrize("precision", ["float64", "float32", "fp32c"])
+def test_small_grids_on_a_part_of_the_sms(few_sms, precision):
+    """Where the launch of all steps is refused for want of resident blocks, the
+    call runs step by step: the fields of the other path."""
+    kw = {"precision": "fp32c"} if precision == "fp32c" else {"dtype": np.dtype(precision).type}
+    sol = []
+    for stream in (few_sms, torch.cuda.current_stream()):
+        s = _solver((44, 33, 57), bcs=OPEN, **kw)
+        s._desc.wait_ns = 200_000_000
+        _random_state(s, e=precision != "fp32c")
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            s._advance(9, 0)
+            s.check_status()
+        torch.cuda.synchronize()
+        sol.append(s)
+    assert _equal(*sol)
+    assert int(sol[0]._sync.abs().sum().item()) == 0

@@ -274,8 +274,8 @@ int wk_comp_step(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_
     const FitParams<double> p = make_params<double>(d, par);
     if (loop_comp_supported(p)) {
       cudaError_t e = launch_loop_comp(d, p, n_steps, step0, st);
-      if (e != cudaSuccess) return wk_fail(-(int)e, "wk_fit_step: %s", cudaGetErrorString(e));
-      return wk_check_launch("wk_fit_step");
+      if (e == cudaSuccess) return wk_check_launch("wk_fit_step");
+      if (!loop_refused(e)) return wk_fail(-(int)e, "wk_fit_step: %s", cudaGetErrorString(e));
     }
   }
   if (!cstencil && (d->kernel == WK_KERNEL_AUTO || d->kernel == WK_KERNEL_TMA)) {

@@ -276,6 +276,15 @@ template <typename T>
 cudaError_t launch_loop(const FitParams<T>& p, int n_steps, long long step0, unsigned* sync,
                         cudaStream_t st);
 
+// A launch of launch_loop or launch_loop_comp refused because its blocks cannot
+// all be resident (a context that is given fewer SMs than the device has):
+// nothing was written, and the call runs step by step.  Clears the error.
+inline bool loop_refused(cudaError_t e) {
+  if (e != cudaErrorCooperativeLaunchTooLarge) return false;
+  (void)cudaGetLastError();
+  return true;
+}
+
 // Two steps per launch (fit_tma2.cu): k_tma2 covers grids whose faces are
 // all PEC-masked and clean, with J = 0 or sigma*E.
 template <typename T>

@@ -124,8 +124,8 @@ int run_fused(const wk_fit_desc* d, int n_steps, long long step0, cudaStream_t s
     const FitParams<T> p = make_params<T>(d, par);
     if (loop_supported<T>(p)) {
       cudaError_t e = launch_loop<T>(p, n_steps, step0, d->sync, st);
-      if (e != cudaSuccess) return wk_fail(-(int)e, "wk_fit_step: %s", cudaGetErrorString(e));
-      return wk_check_launch("wk_fit_step");
+      if (e == cudaSuccess) return wk_check_launch("wk_fit_step");
+      if (!loop_refused(e)) return wk_fail(-(int)e, "wk_fit_step: %s", cudaGetErrorString(e));
     }
   }
   bool use_tma = d->kernel == WK_KERNEL_TMA;
