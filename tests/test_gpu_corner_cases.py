@@ -229,3 +229,37 @@ def test_small_grids_on_a_part_of_the_sms(few_sms, precision):
         sol.append(s)
     assert _equal(*sol)
     assert int(sol[0]._sync.abs().sum().item()) == 0
+
+
+def _cavities(n, precision, shape=(16, 20, 24)):
+    import wakis_b200 as wb
+    sol = []
+    for q in range(n):
+        g = wb.GridFIT3D(-0.008, 0.008, -0.01, 0.01, -0.012, 0.012, *shape, verbose=0)
+        m = np.ones(shape, bool)
+        m[3:13, 4:16, :] = False
+        g.add_solid("wall", m, [1.0, 1.0, 0.5 + 0.05 * q])
+        w = wb.WakeSolver(q=1e-9, sigmaz=3e-3, save=False, verbose=0)
+        kw = {"precision": "fp32c"} if precision == "fp32c" else {"dtype": np.dtype(precision).type}
+        sol.append(wb.SolverFIT3D(g, w, bc_low=OPEN[0], bc_high=OPEN[1], use_stl=True, use_sibc=False,
+                                  bg="vacuum", verbose=0, **kw))
+    return sol
+
+
+@pytest.mark.parametrize("precision,count,form", [("fp32c", 2, "loop"), ("fp32c", 14, "batched"),
+                                                  ("float64", 2, "loop"), ("float64", 6, "graph"),
+                                                  ("float32", 6, "graph")])
+def test_batch_form_by_count_and_its_results(precision, count, form):
+    """The form that is picked, and the wake potentials of single runs whose
+    steps are launched one by one."""
+    from wakis_b200 import batch
+    sol = _cavities(count, precision)
+    b = batch.BatchedWakeSolve(sol, 251, tune=False)
+    assert b.launch == form
+    b.run()
+    ref = _cavities(count, precision)
+    for s, r in zip(sol, ref):
+        r.steps_per_launch = 1
+        r.wakesolve(wakelength=batch.BatchedWakeSolve.wakelength_for(r, 251))
+        assert np.abs(r.wake.WP).max() > 0
+        assert np.array_equal(s.wake.WP_3d, r.wake.WP_3d) and np.array_equal(s.wake.Zx, r.wake.Zx)

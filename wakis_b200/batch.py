@@ -154,10 +154,49 @@ def batched_ok(solvers):
 
 
 def loop_ok(solvers, n_steps):
-    """True when every solver runs n_steps steps of a call in one launch."""
+    """True when every solver, all on one device, runs n_steps steps of a call
+    in one launch."""
     lib = _native.lib()
-    return bool(solvers) and all(lib.wk_fit_one_launch(s._step_desc(), int(n_steps))
-                                 for s in solvers)
+    return (bool(solvers) and all(s.device == solvers[0].device for s in solvers) and
+            all(lib.wk_fit_one_launch(s._step_desc(), int(n_steps)) for s in solvers))
+
+
+def loop_pays(solvers):
+    """True when the instances one after another (launch="loop", for solvers
+    that ``loop_ok`` accepts) take no longer than stepped together.
+
+    In turn, a step costs the sum over the instances: 3.4 us and 1.8 to 2.8 us
+    per 10^5 cells each.  Together, it costs a latency of all and less per
+    instance.  So the line is a count; measured on B200 (us a step of all
+    instances, in turn / together, capture included, 2000 to 3000 steps):
+
+    * against the work list (FP32c), untuned and tuned: 16x16x32 open 8
+      instances 38 / 80 and 59, 16 76 / 80 and 60, 32 152 / 85; 24x24x48 closed
+      8 28 / 71 and 49, 16 56 / 72 and 48; 36x33x61 open 24 120 / 153 and 145, 32
+      160 / 167 and 183; 40x40x80 open 24 157 / 160 and 163, 32 209 / 181 and 177,
+      closed 8 49 / 80 and 59, 16 99 / 87 and 66; 56x56x112 open 24 261 / 287 and
+      328, closed 8 83 / 92 and 83, 16 166 / 125 and 130;
+    * against the graph: FP32c 17x17x32 8 33 / 32, 35x33x61 32 158 / 288,
+      41x40x80 32 243 / 431 (four launches a step there); FP64 16x16x32 open 4
+      16 / 17, 8 32 / 20; 40x40x80 open 4 28 / 29, 8 55 / 51, closed 2 14 / 20, 4
+      27 / 26; 56x56x112 open 4 53 / 68, closed 2 25 / 27, 4 51 / 46; rows that
+      are no multiple of 16 bytes: 33x36x61 FP64 8 44 / 48,
+      FP32 35 / 43, closed 40 / 42 and 34 / 38, 25x24x48 8 34 / 27."""
+    n = len(solvers)
+    cells = sum(s.Nx * s.Ny * s.Nz for s in solvers) / n
+    small = cells < 50000
+    d = solvers[0]._desc
+    closed = bool(d.has_pec) and not d.has_pmc and not any(d.pec_face)
+    odd = any(s.Nx * (8 if s._desc.dtype == _native.WK_F64 else 4) % 16 for s in solvers)
+    if batched_ok(solvers):
+        most = 12 if small else (8 if closed else 24)
+    elif d.dtype == _native.WK_F32C:
+        most = 8 if small or not odd else n
+    elif closed and cells >= 100000:
+        most = 2
+    else:
+        most = 8 if odd and not small else 4
+    return n <= most
 
 
 def autotune_batch(solvers, candidates=BATCH_KC_CANDIDATES, forms=tuple(FORMS), steps=4,
@@ -210,9 +249,11 @@ class BatchedWakeSolve:
     launch: "batched" (the device work list over all instances,
     wk_batch_run, for FP32-compensated instances), "graph" (replayed graph of
     per-instance launches), "loop" (one launch per instance for all its steps)
-    or "auto" (loop when ``loop_ok``: a call with 8 cavities of 40x40x96 to
-    64x64x119 cells and 900 steps took 84 ms, batched 187; else batched when
-    ``batched_ok``).  form:
+    or "auto" (loop when ``loop_ok`` and ``loop_pays``: few small instances; else
+    batched when ``batched_ok``, else graph).  What another form alone reads is
+    not used: form, tiles and chunk are the batched launch's (form or tiles other
+    than "auto" rule the loop out), streams the graph's, tune both of theirs.
+    form:
     the batched launch form, "persistent", "phases" or "auto" (chosen by the
     autotuner; "persistent" without tuning).  tiles: the tile shapes of the
     batched launch, "64x8", "32x16", "fill" (per instance, the shape with
@@ -243,7 +284,7 @@ class BatchedWakeSolve:
         self.timing = {}
         if launch == "auto":
             launch = ("loop" if form == "auto" and tiles == "auto" and
-                      loop_ok(self.solvers, n_steps - 1) else
+                      loop_ok(self.solvers, n_steps - 1) and loop_pays(self.solvers) else
                       "batched" if batched_ok(self.solvers) else "graph")
         elif launch == "loop" and not loop_ok(self.solvers, n_steps - 1):
             raise ValueError("launch='loop' needs grids whose steps run in one launch")
