@@ -263,3 +263,78 @@ def test_batch_form_by_count_and_its_results(precision, count, form):
         r.wakesolve(wakelength=batch.BatchedWakeSolve.wakelength_for(r, 251))
         assert np.abs(r.wake.WP).max() > 0
         assert np.array_equal(s.wake.WP_3d, r.wake.WP_3d) and np.array_equal(s.wake.Zx, r.wake.Zx)
+
+
+@pytest.mark.parametrize("precision", [None, "fp32c"])
+@pytest.mark.parametrize("tune", [False, True])
+def test_graph_of_per_instance_launches(precision, tune):
+    """launch='graph': uneven pillboxes (surface impedance walls among them) on
+    several streams, the step index from the device counter, an odd and an even
+    number of steps after the first; the results of single runs whose steps are
+    launched one by one."""
+    from wakis_b200 import batch
+
+    def boxes():
+        return [batch.build_pillbox(cell=2e-3, precision=precision, **q)[2] for q in (
+            dict(R=0.020, L=0.030, beta=0.9, sigma=1e4), dict(R=0.026, L=0.036, beta=0.6, sigma=3e5),
+            dict(R=0.022, L=0.040, beta=1.0, sigma=2e3))]
+
+    for steps in (600, 601):
+        inst, solo = boxes(), boxes()
+        b = batch.BatchedWakeSolve(inst, steps, launch="graph", streams=4, tune=tune)
+        assert b.launch == "graph"
+        b.run()
+        for s, r in zip(inst, solo):
+            r.steps_per_launch = 1
+            r.wakesolve(wakelength=batch.BatchedWakeSolve.wakelength_for(r, steps))
+            assert r.Nt == steps and np.abs(r.wake.WP).max() > 0
+            assert np.array_equal(s.wake.WP, r.wake.WP) and np.array_equal(s.wake.Z, r.wake.Z)
+            assert np.array_equal(s.E.numpy(), r.E.numpy())
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n,shape", [(80, (12, 10, 90)), (290, (9, 8, 300))])
+def test_one_launch_with_many_materials(dtype, n, shape):
+    """More materials than fit beside the tiles (ids of one and two bytes)."""
+    import wakis_b200 as wb
+    from wakis_b200 import _native
+    sol = []
+    for kernel in ("auto", "cell"):
+        g = wb.GridFIT3D(-0.03, 0.031, -0.02, 0.022, -0.14, 0.143, *shape, verbose=0)
+        for q in range(n):
+            m = np.zeros(shape, bool)
+            m[2:8, 2:7, 4 + q] = True
+            g.add_solid(f"m{q}", m, [1.0 + 0.01 * q, 1.0, 0.1 * (q % 7)])
+        s = wb.SolverFIT3D(g, bc_low=OPEN[0], bc_high=OPEN[1], dtype=dtype, bg=[1.0, 1.0],
+                           use_stl=True, use_sibc=False, verbose=0)
+        s.kernel = kernel
+        assert s._desc.n_mat > (64 if n < 256 else 256)
+        _random_state(s)
+        if kernel == "auto":
+            assert _native.lib().wk_fit_one_launch(s._step_desc(), 9) == 1
+        s._advance(9, 0)
+        s.check_status()
+        sol.append(s)
+    assert _equal(*sol)
+
+
+@pytest.mark.parametrize("precision", ["float64", "float32", "fp32c"])
+def test_one_launch_that_gives_up(precision):
+    """Waits without time: the blocks leave, the host sees the status, the
+    barrier words are zero again and the next run is a run of its own."""
+    kw = {"precision": "fp32c"} if precision == "fp32c" else {"dtype": np.dtype(precision).type}
+    a, b = (_solver((36, 33, 57), bcs=OPEN, **kw) for _ in range(2))
+    _random_state(a, e=False)
+    a._desc.wait_ns = -1
+    a._advance(9, 0)
+    with pytest.raises(RuntimeError, match="gave up waiting"):
+        a.check_status()
+    assert int(a._sync.abs().sum().item()) == 0
+    a._desc.wait_ns = 0
+    for s in (a, b):
+        s.reset_fields()
+        s.step_0, s.nstep = True, 0
+        _random_state(s, e=False)
+        s._advance(9, 0)
+        s.check_status()
+    assert _equal(a, b) and np.abs(a.E.numpy()).max() > 0
