@@ -53,6 +53,7 @@ int wk_validate_fit(const wk_fit_desc* d, const char* where) {
     int a = (i == 4) ? d->id_bytes : (i < 4 ? es : ts);
     if (!aligned(req[i], a)) return wk_fail(WK_E_ALIGN, "%s: %s misaligned", where, names[i]);
   }
+  if (d->sync && !aligned(d->sync, 4)) return wk_fail(WK_E_ALIGN, "%s: sync misaligned", where);
   if (d->par != 0 && d->par != 1) return wk_fail(WK_E_MODE, "%s: par %d", where, d->par);
   if (d->n_mat <= 0) return wk_fail(WK_E_RANGE, "%s: n_mat %d", where, d->n_mat);
   if (d->j_mode < WK_J_ZERO || d->j_mode > WK_J_ARRAY)
