@@ -428,11 +428,16 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
   bool ok = true;
   int pl = pstart;
   const long long lim = loop_wait_ns(p.wait_ns);   // step-loop waits; the drain keeps kWaitNs
+  // LATE: boxes and tables are formed after the H phase, while the tile warps
+  // compute E: the float H phase is so short that it waits for warp 9
+  // (223x177x400: 320 us a step against 330), the double one is not, and the
+  // boxes then arrive late (149x131x301: 177 us against 165)
+  constexpr bool LATE = GRP && sizeof(T) == 4;
   for (; pl < k1; pl++) {
     cp_async_wait<1>();          // this thread's row entry of plane pl
     bool got = true;
     if (prod) got = wait_e(pl, lim) && wait_e(pl + 1, lim) && wait_h(pl, lim);
-    if (GRP && issue_we && pl + 1 >= Nz - 1) {
+    if (GRP && ZFULL && issue_we && pl + 1 >= Nz - 1) {
       // the top plane arrived as E(pl) at the start of a chunk, else as E(pl+1)
       __syncwarp();
       const int se2 = se == kES - 1 ? 0 : se + 1;
@@ -440,22 +445,17 @@ k_tma(FitParams<T> p, const __grid_constant__ TmaMaps maps, long long step, int 
         if (pl == pstart) patch(pl, Eb + se * 3 * SE, etab + se * 3 * S::BY, S::BY, S::TX + 2, p.E_in);
         patch(pl + 1, Eb + se2 * 3 * SE, etab + se2 * 3 * S::BY, S::BY, S::TX + 2, p.E_in);
       }
-      // H's table was written by warp 8 (LATE: since the last block barrier)
-      if (pl == Nz - 1) asm volatile("bar.sync 1, 64;" ::: "memory");
+      // LATE: warp 8 has written H's table since the last block barrier
+      if (LATE && pl == Nz - 1) asm volatile("bar.sync 1, 64;" ::: "memory");
       patch(pl, Hb + sh * 3 * SH, htab + sh * 3 * S::HBY, S::HBY, S::TX + 1, p.H_in);
-    } else if (GRP && issue_wh && pl == Nz - 1) {
+    } else if (LATE && ZFULL && issue_wh && pl == Nz - 1) {
       __syncwarp();
       asm volatile("bar.sync 1, 64;" ::: "memory");    // warps 8 and 9
     }
     ok = __syncthreads_and(got);
     if (!ok) break;
     const bool prologue = pl == pstart;
-    // the slots of E(pl-1) and H(pl-1) are free: every thread finished plane
-    // pl-1.  LATE: boxes and tables are formed after the H phase, while the tile
-    // warps compute E: the float H phase is so short that it waits for warp 9
-    // (223x177x400: 320 us a step against 330), the double one is not, and the
-    // boxes then arrive late (149x131x301: 177 us against 165)
-    constexpr bool LATE = GRP && sizeof(T) == 4;
+    // the slots of E(pl-1) and H(pl-1) are free: every thread finished plane pl-1
     auto issue_next = [&]() {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       if (issue_we && pl + kES - 1 <= k1) issue_e(pl + kES - 1);
