@@ -814,24 +814,18 @@ static bool tma_narrow(const FitParams<T>& p, bool grp) {
 }
 
 // One step with the TMA kernel in the mode the faces allow (see k_tma), on
-// 64x8 tiles (rows 8), 32x16 tiles (rows 16) or the better of the two (rows 0).
-template <typename T>
-cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
-                       int rows) {
+// tiles of `w32` columns, GRP as the rows need it.
+template <typename T, bool GRP>
+cudaError_t launch_tma_rows(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
+                            bool w32) {
   const bool sm_table = p.n_mat <= kMatSmem && p.id_bytes == 1;
   const int jm = p.j_mode == WK_J_SIGMA_E ? 1 : (p.j_mode == WK_J_ARRAY ? 2 : 0);
   const int mode = tma_mode(p);
   const bool desc = p.h_desc != 0;
-  const bool grp = row_group(p) > 1;
-  const bool w32 = rows == 16 || (rows == 0 && tma_narrow(p, grp));
 #define WK_TMA_WIDTH(SMV, JMV, MV, DV)                                                \
   {                                                                                   \
-    if (grp) {                                                                        \
-      if (w32) return launch_tma_variant<T, SMV, JMV, MV, DV, true, 32>(p, step, st, KC); \
-      return launch_tma_variant<T, SMV, JMV, MV, DV, true, 64>(p, step, st, KC);      \
-    }                                                                                 \
-    if (w32) return launch_tma_variant<T, SMV, JMV, MV, DV, false, 32>(p, step, st, KC); \
-    return launch_tma_variant<T, SMV, JMV, MV, DV, false, 64>(p, step, st, KC);       \
+    if (w32) return launch_tma_variant<T, SMV, JMV, MV, DV, GRP, 32>(p, step, st, KC); \
+    return launch_tma_variant<T, SMV, JMV, MV, DV, GRP, 64>(p, step, st, KC);         \
   }
 #define WK_TMA_MODES(SMV, JMV, DV)                                                    \
   {                                                                                   \
@@ -852,6 +846,32 @@ cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, i
   return cudaErrorInvalidValue;
 }
 
+// The kernel's 288 instances are compiled in four units, one per type and row
+// form (fit_tma_f32.cu, fit_tma_rows.cu and fit_tma_rows_f32.cu set WK_TMA_PART
+// and include this file); this one also holds what they share.
+#ifdef WK_TMA_PART
+template cudaError_t launch_tma_rows<WK_TMA_PART>(const FitParams<WK_TMA_TYPE>&, long long,
+                                                  cudaStream_t, int, bool);
+#else
+template cudaError_t launch_tma_rows<double, false>(const FitParams<double>&, long long,
+                                                    cudaStream_t, int, bool);
+extern template cudaError_t launch_tma_rows<double, true>(const FitParams<double>&, long long,
+                                                          cudaStream_t, int, bool);
+extern template cudaError_t launch_tma_rows<float, false>(const FitParams<float>&, long long,
+                                                          cudaStream_t, int, bool);
+extern template cudaError_t launch_tma_rows<float, true>(const FitParams<float>&, long long,
+                                                         cudaStream_t, int, bool);
+
+// On 64x8 tiles (rows 8), 32x16 tiles (rows 16) or the better of the two (rows 0).
+template <typename T>
+cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
+                       int rows) {
+  const bool grp = row_group(p) > 1;
+  const bool w32 = rows == 16 || (rows == 0 && tma_narrow(p, grp));
+  return grp ? launch_tma_rows<T, true>(p, step, st, KC, w32)
+             : launch_tma_rows<T, false>(p, step, st, KC, w32);
+}
+
 template bool tma_pitch<double>(const FitParams<double>&);
 template bool tma_pitch<float>(const FitParams<float>&);
 template bool tma_supported<double>(const FitParams<double>&);
@@ -859,5 +879,6 @@ template bool tma_supported<float>(const FitParams<float>&);
 template cudaError_t launch_tma<double>(const FitParams<double>&, long long, cudaStream_t, int,
                                         int);
 template cudaError_t launch_tma<float>(const FitParams<float>&, long long, cudaStream_t, int, int);
+#endif
 
 }  // namespace wk
