@@ -338,3 +338,29 @@ def test_one_launch_that_gives_up(precision):
         s._advance(9, 0)
         s.check_status()
     assert _equal(a, b) and np.abs(a.E.numpy()).max() > 0
+
+
+@pytest.mark.parametrize("precision", ["float64", "float32", "fp32c"])
+@pytest.mark.parametrize("shape,bcs", [((36, 33, 57), OPEN), ((33, 20, 41), PEC), ((37, 21, 40), OPEN)])
+def test_one_launch_calls_between_single_steps(precision, shape, bcs):
+    """Calls that run in one launch, single steps and host traffic in turn: what
+    one leaves in either buffer is what the next one needs."""
+    kw = {"precision": "fp32c"} if precision == "fp32c" else {"dtype": np.dtype(precision).type}
+    sol, out = [], []
+    for spl in (0, 1):
+        s = _solver(shape, bcs=bcs, **kw)
+        s.steps_per_launch = spl
+        _random_state(s, e=False)
+        rng = np.random.default_rng(5)
+        ez = []
+        for n in (9, 1, 8, 3, 1, 1, 12):
+            s._advance(n, s.nstep)
+            lines = 1e-3 * rng.standard_normal((7, s.Nz))
+            buf = torch.empty((7, 9, s.Nz), dtype=s._cap_dtype).pin_memory()
+            s.run_with_io(torch.as_tensor(lines).to(s._cap_dtype).pin_memory(), buf)
+            ez.append(buf.clone())
+        s.check_status()
+        sol.append(s)
+        out.append(ez)
+    assert _equal(*sol) and all(torch.equal(a, b) for a, b in zip(*out))
+    assert np.abs(sol[0].E.numpy()).max() > 0
