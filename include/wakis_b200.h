@@ -140,8 +140,9 @@ typedef struct wk_fit_desc {
    * full-domain TMA kernels then skip the PEC column masks of the H rows,
    * which would only replace +0 by +0.  0 (the default) always masks.      */
   int faces_clean;
-  /* Bound of each mbarrier wait in the step loop of the TMA kernels, in
-   * nanoseconds of the GPU's global timer; 0 (the default) = 100 ms.  A
+  /* Bound of each mbarrier wait in the step loop of the TMA kernels and of
+   * each grid-barrier wait of the one-launch steps (sync), in nanoseconds of
+   * the GPU's global timer; 0 (the default) = 100 ms and 2 s.  A
    * negative value makes the first wait give up at once: the block then
    * records the timeout in *status, waits with the default bound for the
    * loads it issued and returns (a test of the timeout path, which leaves
@@ -149,12 +150,13 @@ typedef struct wk_fit_desc {
   long long wait_ns;
   /* Steps per launch of the TMA schedule: 2 = two steps per launch
    * (temporal blocking, k_tma2) where that kernel applies (every face
-   * PEC-masked, faces_clean, J = 0 without conductivity or sigma*E with it,
-   * no step_dev) and n_steps >= 4, else one; 1 = always one; 0 (the
-   * default) = the faster on B200 for the state type: one step per launch
-   * for FP64 and FP32 (k_tma2 halves the DRAM bytes but issues more
-   * instructions per cell at a lower occupancy).  The result and its buffer
-   * parity do not depend on it.                                            */
+   * PEC-masked, faces_clean, rows and components of a multiple of 16 bytes,
+   * J = 0 without conductivity or sigma*E with it, no step_dev) and n_steps
+   * >= 4, else one; 1 = always one; 0 (the default) = the faster on B200:
+   * all steps of a call on small grids (sync), else one step per launch
+   * (k_tma2 halves the DRAM bytes but issues more instructions per cell at
+   * a lower occupancy).  The result and its buffer parity do not depend on
+   * it.                                                                    */
   int steps_per_launch;
   /* WK_F32C only.  0 (the default): the rows read the float parts v of the
    * neighbouring state and sum in float; the compensated add then keeps

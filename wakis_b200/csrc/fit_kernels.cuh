@@ -268,8 +268,8 @@ template <typename T>
 cudaError_t launch_tma(const FitParams<T>& p, long long step, cudaStream_t st, int KC,
                        int rows);
 
-// All steps of a call in one launch, for small grids (fit_loop.cu): the grid
-// fits the row factors kept in shared memory; every dimension >= 2.
+// All steps of a call in one launch, for small grids (fit_loop.cu): those whose
+// state fits the shared memory of the SMs; every dimension >= 5.
 template <typename T>
 bool loop_supported(const FitParams<T>& p);
 template <typename T>

@@ -81,17 +81,19 @@ struct TmaMaps {
 };
 
 // Row groups (GRP): a row pitch that is no multiple of 16 bytes becomes one when
-// kGroup = 2 or 4 rows are taken together, so the rows of a field (all three
+// row_group() = 2 or 4 rows are taken together, so the rows of a field (all three
 // components, in flat order) form a 2-D tensor of `group` Nx wide super-rows,
 // and a tile's rows of each residue (flat row mod group) are one box of it.
-// Per component a slot holds `group` boxes of grp_rows() rows; a row starts at ext column 0 rounded down to 16 bytes.  The offset of ext
-// column 0 of every (component, ext row) is tabulated per slot by warp 9 when
-// it issues the boxes (the residues of a plane's rows change with the plane).
+// Per component a slot holds `group` boxes of grp_rows() rows; a row starts at
+// ext column 0 rounded down to 16 bytes.  The offset of ext column 0 of every
+// (component, ext row) is tabulated per slot by the warp that issues the boxes, 9
+// for E and 8 for H (the residues of a plane's rows change with the plane).
 // The rows past the last whole super-row are copied by hand.
-// Measured on B200 against the two-pass schedule (us a step): 149x131x301 FP64
-// with open ends 288 / 165, 223x177x200 FP64 324 / 195, 81x77x160 FP64 closed
-// 68 / 35, 101x99x203 FP32 79 / 60, 223x177x400 FP32 454 / 320; one bulk copy
-// per row instead of boxes of rows took 239 and 417 us on the first and last.
+// Measured on B200, the two-pass schedule / this (us a step): 149x131x301 FP64
+// with open ends 285 / 149, 223x177x200 FP64 open 322 / 185, 81x77x160 FP64 closed
+// 67 / 35, 101x99x203 FP32 closed 77 / 57, 223x177x400 FP32 open 448 / 311, closed
+// 449 / 321; one bulk copy per row instead of boxes of rows took 239 and 417 us
+// on the first and last, where boxes took 165 and 320 then.
 constexpr int grp_rows(int rows, int group) { return (rows + group - 1) / group; }
 template <typename T>
 constexpr int kGroupMax = sizeof(T) == 8 ? 2 : 4;

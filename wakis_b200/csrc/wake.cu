@@ -1,7 +1,7 @@
 // Wake potential and impedance kernels (sm_100a) and their C-ABI launchers.
 //
 // wk_wake_potential  calc_long_WP_3d / calc_long_WP (wakis/wakeSolver.py:
-//                    310-554): one thread per s sample, the transverse
+//                    310-554): a block per 32 s samples, the transverse
 //                    positions in upstream order with the running-sum
 //                    carry-over, and the z sum in upstream's sequential
 //                    order, so WP matches upstream value for value.
@@ -53,10 +53,14 @@ __device__ __forceinline__ Idx wake_column(const WakeArgs& g, const double* __re
 // The columns, two divisions each, are formed once per (sample, z) and kept in
 // shared memory for the other windows when they fit (COLS).  Idx: long long
 // where a column or a term's number does not fit an int.
-// Bound by the chain and the history's read.  On B200, 9 windows of nz = 400,
-// ns = 11700, FP64: 272 us (345 MB), nz = 120, ns = 4700 55 us; 2632 with one thread per sample
-// that formed the column of every term and waited for its entry, 1158 with one
-// warp per block doing both parts; 4 terms per warp and chunk 257 and 85 us.
+// Bound by the latency of the history: two entries of two chunks are on their way
+// in a forming thread, and a barrier ends every 16 terms, so that a term takes
+// some 140 cycles of a sample's 3600, of which the dependent add about ten; the
+// history's read is at 1.3 TB/s.  On B200, 9 windows of nz = 400, ns = 11700,
+// FP64: 267 us (345 MB), nz = 120, ns = 4700 54 us; nz = 400, ns = 10618: 2632 with
+// one thread per sample that formed the column of every term and waited for its
+// entry, 1158 with one warp per block doing both parts; 4 terms per warp and chunk
+// 257, and 85 for nz = 120.
 constexpr int kWakeProd = 8, kWakeEach = 2, kWakeChunk = kWakeProd * kWakeEach;
 template <typename H, bool COLS, typename Idx>
 __global__ void __launch_bounds__((kWakeProd + 1) * 32)
@@ -349,7 +353,7 @@ __device__ __forceinline__ Pw4 pw_warp4(const double* const* a, int n, int lane)
 
 // Positions (+1,0) (-1,0) (0,+1) (0,-1) are w = 7, 1, 5, 3 of the 3x3 block;
 // one warp forms the four prefix integrals of a sample.  O(ns^2) adds in
-// numpy's order.  On B200, ns = 11700: 151 us; 1052 with one thread
+// numpy's order.  On B200, ns = 10618: 149 us; 1052 with one thread
 // per sample, 623 with one node per lane (32 lines a load).
 constexpr int kTransWarps = 8;
 __global__ void __launch_bounds__(kTransWarps * 32)
@@ -553,8 +557,8 @@ __global__ void k_trans_final(const double* __restrict__ WP3d, int ns, int seg,
 // about T + len / T exponentials instead of len; the exponentials w^(T a) come
 // from shared memory, kDftChunk at a time.  Fixed-shape tree reduction
 // (deterministic).  40 registers, six blocks an SM (without the bound 42: five,
-// 4 signals 47.2 us for 45.1).  On B200, 984 bins of 11700 samples: 2 signals 25 us,
-// 3 signals 34 us; 127 us on average with one exponential per term.
+// 4 signals 47.2 us for 45.1).  On B200, 984 bins of 11700 samples, 4 signals: 45
+// us, 209 with one exponential per term.
 constexpr int kDftThreads = 256, kDftChunk = 256;
 // cos and sin of 2 pi m n / N, the angle brought within an eighth of a turn by
 // exact integer quarter turns first (so that its rounding, relative to a small

@@ -202,7 +202,8 @@ class SolverFIT3D(RoutinesMixin):
         self.tile = (0, 0)
         # wk_fit_desc.steps_per_launch: 2 runs pairs of steps as one launch of
         # the temporal-blocking kernel where it applies, 1 one step per
-        # launch, 0 the faster on B200 (one step per launch)
+        # launch, 0 the faster on B200 (all steps of a call on small grids,
+        # else one step per launch)
         self.steps_per_launch = 0
         # precision='fp32c' only: True forms every increment from the full
         # (float + compensation) neighbour values with error-free float
