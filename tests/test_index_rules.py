@@ -49,3 +49,21 @@ int main() {
   return 0;
 }
 """)
+
+
+def test_barrier_count_of_a_call_with_very_many_steps(tmp_path):
+    """The arrivals of a grid barrier against their target where both pass 2^32."""
+    _host_program(tmp_path, """
+#include "fit_loop.cuh"
+int main() {
+  for (unsigned blocks : {1u, 7u, 148u, 160u})
+    for (long long step : {1LL, 2LL, 29020049LL, 29020050LL, 29020051LL, 2147483647LL}) {
+      const long long target = step * blocks;
+      for (long long behind = -(long long)blocks; behind <= (long long)blocks; behind++) {
+        const long long count = target - behind;
+        if (wk::loop_arrived((unsigned)count, (unsigned)target) != (count >= target)) return 1;
+      }
+    }
+  return 0;
+}
+""")

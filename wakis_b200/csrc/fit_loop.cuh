@@ -43,14 +43,19 @@ __device__ __forceinline__ void red_release(unsigned* a) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a) : "memory");
 }
 
+// Whether a count that wraps at 2^32 (29 million steps of 148 blocks) has reached
+// the target, from which it is never further than a grid.
+__host__ __device__ __forceinline__ bool loop_arrived(unsigned count, unsigned target) {
+  return (int)(count - target) >= 0;
+}
 // Thread 0: wait until `target` arrivals were counted.  False when the wait
 // ran out or another block gave up.
 __device__ __forceinline__ bool loop_wait(unsigned* sync, unsigned target, long long limit_ns) {
   if (limit_ns < 0) return false;
-  if (ld_acquire(sync + kSyncCount) >= target) return true;
+  if (loop_arrived(ld_acquire(sync + kSyncCount), target)) return true;
   const unsigned long long t0 = globaltimer_ns();
   for (long long it = 0; it < kWaitPolls; it++) {
-    if (ld_acquire(sync + kSyncCount) >= target) return true;
+    if (loop_arrived(ld_acquire(sync + kSyncCount), target)) return true;
     if ((it & 63) == 63 && (ld_acquire(sync + kSyncAbort) != 0 ||
                             (long long)(globaltimer_ns() - t0) > limit_ns))
       return false;
