@@ -140,14 +140,13 @@ def test_dft_bins_of_infinite_signals(length, N, at, value):
             assert np.array_equal(got[0, m, part], want, equal_nan=True), (m, part)
 
 
-@pytest.mark.parametrize("nz", [1, 5])
+@pytest.mark.parametrize("nz", [1, 2])
 def test_wake_potential_of_a_history_past_int_columns(nz):
     """More than 2^31 columns (FP32, 8.6 GB a row): the entries of the last
     ones are the ones read."""
     from wakis_b200 import _native
-    nt, rows, ns, dt = 2 ** 31 + 9, 1, 8 - nz + 1, 1e-12
-    hist = torch.empty(rows * nt * (1 if nz == 1 else 5), dtype=torch.float32, device="cuda")
-    rows = hist.numel() // nt
+    nt, rows, ns, dt = 2 ** 31 + 9, nz, 8 - nz + 1, 1e-12
+    hist = torch.empty(rows * nt, dtype=torch.float32, device="cuda")
     order = torch.arange(nt - 8, nt, dtype=torch.int64, device="cuda")
     rng = np.random.default_rng(1)
     vals = rng.standard_normal((rows, 8)).astype(np.float32)
@@ -167,6 +166,8 @@ def test_wake_potential_of_a_history_past_int_columns(nz):
     for k in range(nz):
         ref += vals[k, np.arange(ns) + k].astype(np.float64)
     assert np.array_equal(WP.cpu().numpy()[0], ref)
+    del hist
+    torch.cuda.empty_cache()
 
 
 @pytest.mark.parametrize("ns", [65535, 65536, 65537, 131073, 200003])
